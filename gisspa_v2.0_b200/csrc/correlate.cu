@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(NW * 32, MINB)
                                               (unsigned)(0xFFFFFFFFu - (unsigned)barg[s][i][h]));
           }
           if constexpr (EPI == EPI_SUMMAX)
-            atomicMax(a.peak + pix + h, (unsigned long long)float_key(best[s][i][h] * inv) << 32);
+            atomicMax(a.peak32 + pix + h, float_key(best[s][i][h] * inv));
         }
       }
     }

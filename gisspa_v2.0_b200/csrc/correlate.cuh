@@ -24,7 +24,7 @@ enum Epilogue : int {
   EPI_TOPK = 2,    // one sweep: S1, S2 and per-pixel max c with its (angle, template)
   EPI_NONORM = 3,  // norm_type=0: per pair peak (border zeroed), sum, sum of squares of CC
   EPI_MAP = 4,     // write c maps (tests and the no-scratch entry point)
-  EPI_SUMMAX = 5   // sweep 1 of a pruned search: S1, S2 and the per-pixel max c (peak key, no index)
+  EPI_SUMMAX = 5   // sweep 1 of a pruned search: S1, S2 and the per-pixel max c (no index)
 };
 
 // A picked chunk (or, for EPI_NONORM, nothing: per-pair reductions go to nn_*).
@@ -78,6 +78,8 @@ struct CorrArgs {
   // (float_key(c) << 32) | (0xFFFFFFFF - k), 0 = none yet: an integer max keeps the larger c
   // and, on ties, the lower k (the first one a single sweep meets)
   unsigned long long* peak;
+  // EPI_SUMMAX: per pixel float_key of the best correlation, 0 = none yet
+  unsigned* peak32;
   // EPI_CHUNK
   const float2* musig;      // [W][L][L] (mu, 1/sigma or 0)
   float thresh;
@@ -143,6 +145,27 @@ size_t engine_counter_ints();
 void engine_launch(int spec, int epi, const float2* I, const void* T, const EngineBatch& A, const EngineBatch& B,
                    const CorrArgs& b_args, int* ctr, bool chained, const float2* twL, const float2* twNZ,
                    cudaStream_t s);
+
+// ---- sweep 1 with two templates per transform (corr_pair.cu): EPI_SUM, EPI_SUMMAX and EPI_TOPK
+// at window sizes 256, 320 and 512.  Adds the sums of squares and the maxima to the state; the
+// plain sums come from pair_sum_finish.
+bool pair_supported(int L, int epi);
+// Windows and (an even number of) templates per launch.
+void pair_batch(int L, int W, int nt, int& D, int& E);
+// Bytes of one template pair's spectra, and of the running sum of all templates' spectra (zeroed
+// by the caller before a sweep).
+size_t pair_spectrum_bytes(int L, int spec);
+size_t pair_sum_bytes(int L);
+// Pairs' spectra of one angle from the rotated templates' half spectra X[n][kx][ky] and their
+// sums (as finalize_spectra), added to the running sum as well.
+void pair_spectra(const float2* X, int nt, int L, const double* sums, int spec, void* out, double base, void* tsum,
+                  cudaStream_t s);
+// The half spectrum (FP32) of the sum of every template-rotation since tsum was zeroed.
+void pair_sum_finish(const void* tsum, int L, float2* out, cudaStream_t s);
+// Column and row pass of cl.D templates from a.n0 (even) and cl.E windows from a.b0.
+// Q: D rounded up to even, x E x L x L / 2 float2.
+void pair_launch(const CorrLaunch& cl, const float2* I, const void* T, float2* Q, const CorrArgs& args,
+                 const float2* twL, cudaStream_t s, cudaEvent_t* ev = nullptr);
 
 // Number of pass A shapes compiled for a window size.
 int pass_a_variants(int L);

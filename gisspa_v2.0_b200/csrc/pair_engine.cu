@@ -200,7 +200,7 @@ __device__ __forceinline__ bool engine_row(const CorrArgs& a, int e, int y, floa
                                             (unsigned)(0xFFFFFFFFu - (unsigned)barg[i][h]));
         }
         if constexpr (EPI == EPI_SUMMAX)
-          atomicMax(a.peak + pix + h, (unsigned long long)float_key(best[i][h] * inv) << 32);
+          atomicMax(a.peak32 + pix + h, float_key(best[i][h] * inv));
       }
     }
   }

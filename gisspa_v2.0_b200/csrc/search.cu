@@ -167,7 +167,7 @@ __global__ void peak_flip_kernel(const unsigned long long* __restrict__ in, long
 // correlation that reaches the threshold less the margin at any live pixel of the window: a
 // pair whose maximum over the window stays below it holds no pick either.
 constexpr float kAliveMargin = 1e-3f;
-__global__ void row_alive_kernel(const unsigned long long* __restrict__ peak, const float2* __restrict__ ms, int l,
+__global__ void row_alive_kernel(const unsigned* __restrict__ peak, const float2* __restrict__ ms, int l,
                                  long long rows, float thresh, unsigned char* __restrict__ alive,
                                  unsigned char* __restrict__ alive_win, unsigned* __restrict__ count,
                                  unsigned* __restrict__ creq) {
@@ -181,10 +181,10 @@ __global__ void row_alive_kernel(const unsigned long long* __restrict__ peak, co
   unsigned req = 0xFFFFFFFFu;  // float_key of +inf and above: no bar yet
   const double t = (double)thresh - (double)kAliveMargin;
   for (int x = lane; x < l; x += 32) {
-    const unsigned long long pk = peak[base + x];
+    const unsigned pk = peak[base + x];
     if (!pk) continue;
     const float2 m = ms[base + x];
-    const float z = (key_float((uint32_t)(pk >> 32)) - m.x) * m.y;
+    const float z = (key_float(pk) - m.x) * m.y;
     if (z >= thresh - kAliveMargin) {
       hit = true;
       // c reaches z = t where c = mu + t / (1 / sigma), rounded down; with 1 / sigma = 0 every c
@@ -372,9 +372,9 @@ void window_spectra(Ctx& c, const float* img, int nx, int ny, const std::vector<
 
 // RotateTemplate (norm.cu:479-521): rotate, mask, (x - mean)/sqrt(var), FFT / l^2.
 // st (optional): take the angle from device memory (graph replays); theta is then unused.
-// Rotation by theta, forward transform and scaling of n prepared templates (src) into spectra
-// (dst, in the storage type of the search's precision).
-void spectra_of(Ctx& c, float theta, const float* src, int n, void* dst, const AngleState* st) {
+// Rotation by theta and forward transform of n prepared templates (src): half spectra in rot_tmp,
+// the rotated templates' sums in rsums.
+void rotated_spectra(Ctx& c, float theta, const float* src, int n, const AngleState* st) {
   gisspa_handle* h = c.h;
   const int l = c.l, nt = h->nt, hs = l / 2 + 1;
   const double rad = (double)theta * kRefPi / 180.0;
@@ -386,7 +386,14 @@ void spectra_of(Ctx& c, float theta, const float* src, int n, void* dst, const A
   h->fft.rows(rot, (long long)n * l, l, -1, 1.f, c.s);
   h->fft.transpose(rot, rtmp, n, l, l, c.s, hs);
   h->fft.rows(rtmp, (long long)n * hs, l, -1, 1.f, c.s);
-  finalize_spectra(rtmp, n, l, sums, h->cfg.spectrum_precision, dst, 1.0 / (double)c.L2, c.s);
+}
+
+// The same, scaled into spectra (dst, in the storage type of the search's precision).
+void spectra_of(Ctx& c, float theta, const float* src, int n, void* dst, const AngleState* st) {
+  gisspa_handle* h = c.h;
+  rotated_spectra(c, theta, src, n, st);
+  finalize_spectra(h->rot_tmp.as<float2>(), n, c.l, h->rsums.as<double>(), h->cfg.spectrum_precision, dst,
+                   1.0 / (double)c.L2, c.s);
 }
 
 void template_spectra_at(Ctx& c, float theta, const AngleState* st = nullptr) {
@@ -589,6 +596,94 @@ TuneChoice autotune(Ctx& c, int epi, const float2* I, int W, const void* T, int 
   return best;
 }
 
+// Whether a sweep runs with two templates per transform (corr_pair.cu): every sweep 1 that it is
+// compiled for, unless the configuration fixes the one-template kernels' launch shape or asks
+// for the tensor-core passes.
+bool sweep_paired(const gisspa_config& cfg, int l, int epi) {
+  return pair_supported(l, epi) && cfg.template_batch == 0 && cfg.window_batch == 0 &&
+         !(cfg.tensor_cores && cfg.spectrum_precision == GISSPA_SPEC_FP16 && l == 512);
+}
+
+// One angle of a paired sweep 1: template pairs' spectra (added to the running sum), then every
+// (window, template) pair.
+long long pair_angle(Ctx& c, float theta, const AngleState* st, int epi, int W, CorrArgs args) {
+  gisspa_handle* h = c.h;
+  const int l = c.l, nt = h->nt, spec = h->cfg.spectrum_precision;
+  rotated_spectra(c, theta, h->prep_real.as<float>(), nt, st);
+  void* T = h->tpair.ensure(pair_spectrum_bytes(l, spec) * ((nt + 1) / 2));
+  pair_spectra(h->rot_tmp.as<float2>(), nt, l, h->rsums.as<double>(), spec, T, 1.0 / (double)c.L2,
+               h->tsum.as<void>(), c.s);
+  int D = 1, E = 1;
+  pair_batch(l, W, nt, D, E);
+  float2* Q = buf<float2>(h->Q, (size_t)D * E * (l / 2) * l);
+  const float2* twL = h->fft.twiddles(l);
+  args.err = h->dev_err.as<unsigned>();
+  args.Q = Q;
+  long long pairs = 0, launches = 0, dsum = 0;
+  const int seq = (!h->capturing && h->n_seqs < gisspa_handle::kSeqs) ? h->n_seqs++ : -1;
+  if (seq >= 0) GISSPA_CUDA(cudaEventRecord(h->qev[seq][0], c.s));
+  for (int n0 = 0; n0 < nt; n0 += D)
+    for (int b0 = 0; b0 < W; b0 += E) {
+      CorrLaunch cl{l, std::min(E, W - b0), std::min(D, nt - n0), spec, epi};
+      cl.chained = launches > 0;
+      args.b0 = b0;
+      args.n0 = n0;
+      args.D = cl.D;
+      cudaEvent_t* ev = nullptr;
+      if (h->cfg.cuda_graphs == 0 && (h->launch_index++ & 15) == 0 && h->n_samples < gisspa_handle::kSamples &&
+          !h->capturing) {
+        ev = h->sev[h->n_samples];
+        h->sample_pairs[h->n_samples] = cl.D * cl.E;
+        h->sample_d[h->n_samples] = cl.D;
+        ++h->n_samples;
+      }
+      pair_launch(cl, h->ispec.as<float2>(), T, Q, args, twL, c.s, ev);
+      pairs += (long long)cl.D * cl.E;
+      dsum += cl.D;
+      ++launches;
+    }
+  if (seq >= 0) {
+    GISSPA_CUDA(cudaEventRecord(h->qev[seq][1], c.s));
+    h->seq_launches[seq] = launches;
+    h->seq_pairs[seq] = pairs;
+    h->seq_d[seq] = dsum;
+    h->seq_pruned[seq] = false;
+  }
+  h->st.pass_a_variant = h->st.pass_b_variant = 0;
+  return pairs;
+}
+
+__global__ void add_map_kernel(const float* __restrict__ map, long long n, double* __restrict__ S) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) S[i] += (double)map[i];
+}
+
+// The sum over a paired sweep's correlations at every window pixel, added to S1: correlation is
+// linear in the template, so it is one correlation per window with the sum of the spectra of all
+// template-rotations (accumulated in FP64), instead of one addition per pixel and pair.
+void pair_sums(Ctx& c, int W, double* S1) {
+  gisspa_handle* h = c.h;
+  const int l = c.l;
+  float2* spec = buf<float2>(h->tsum_spec, (size_t)(l / 2 + 1) * l);
+  pair_sum_finish(h->tsum.as<void>(), l, spec, c.s);
+  const int E = std::min(W, 32);
+  float* map = buf<float>(h->sum_map, (size_t)E * c.L2);
+  CorrArgs args{};
+  args.Q = buf<float2>(h->Q, (size_t)E * (l / 2) * l);
+  args.err = h->dev_err.as<unsigned>();
+  args.D = args.nt_real = args.nt_total = 1;
+  args.map_out = map;
+  for (int b0 = 0; b0 < W; b0 += E) {
+    const int e = std::min(E, W - b0);
+    args.b0 = b0;
+    correlate_launch(CorrLaunch{l, e, 1, GISSPA_SPEC_FP32, EPI_MAP}, h->ispec.as<float2>(), spec, h->Q.as<float2>(),
+                     args, h->fft.twiddles(l), h->fft.twiddles(l / 2), c.s);
+    const long long n = (long long)e * c.L2;
+    add_map_kernel<<<ceil_div(n, 256), 256, 0, c.s>>>(map, n, S1 + (size_t)b0 * c.L2);
+    GISSPA_LAUNCH_CHECK();
+  }
+}
+
 // One correlation sweep at one angle over every (window, template) pair.
 long long correlate_all(Ctx& c, int epi, const float2* I, int W, const void* T, int nt, CorrArgs args, int D, int E) {
   gisspa_handle* h = c.h;
@@ -787,6 +882,7 @@ std::vector<unsigned char> angle_graph_key(Ctx& c, const NormRun& r, int epi) {
                         (const void*)h->tspec.as<void>(), (const void*)h->ispec.as<void>(),
                         (const void*)h->Q.as<void>(), (const void*)h->gen_z.as<void>(),
                         (const void*)h->gen_x.as<void>(), (const void*)a.S1, (const void*)a.S2, (const void*)a.peak,
+                        (const void*)a.peak32, (const void*)h->tpair.as<void>(), (const void*)h->tsum.as<void>(),
                         (const void*)a.musig, (const void*)a.skip.rows, (const void*)a.skip.windows,
                         (const void*)a.skip.pairs, (const void*)a.pair_max,
                         (const void*)a.offx, (const void*)a.offy,
@@ -795,6 +891,14 @@ std::vector<unsigned char> angle_graph_key(Ctx& c, const NormRun& r, int epi) {
                         (const void*)h->angle_cur.as<void>()})
     key_put(k, p);
   return k;
+}
+
+// Template spectra of one angle and its correlation sweep (r.args holds the angle).
+long long one_angle(Ctx& c, NormRun& r, int epi, float theta, const AngleState* st) {
+  gisspa_handle* h = c.h;
+  if (sweep_paired(h->cfg, c.l, epi)) return pair_angle(c, theta, st, epi, r.W, r.args);
+  template_spectra_at(c, theta, st);
+  return correlate_all(c, epi, h->ispec.as<float2>(), r.W, h->tspec.as<void>(), h->nt, r.args, r.D, r.E);
 }
 
 // The captured graph of one angle of this sweep (captured on first use, and again whenever its
@@ -827,8 +931,7 @@ AngleGraph& angle_graph(Ctx& c, NormRun& r, int epi) {
   try {
     angle_select_kernel<<<1, 1, 0, c.s>>>(h->angle_table.as<AngleState>(), h->angle_cursor.as<int>(), cur);
     GISSPA_LAUNCH_CHECK();
-    template_spectra_at(c, 0.f, cur);
-    pairs = correlate_all(c, epi, h->ispec.as<float2>(), r.W, h->tspec.as<void>(), h->nt, r.args, r.D, r.E);
+    pairs = one_angle(c, r, epi, 0.f, cur);
   } catch (...) {
     h->capturing = false;
     r.args.angle_state = nullptr;
@@ -861,10 +964,9 @@ void run_angles(Ctx& c, NormRun& r, int epi, int a0, int a1) {
   gisspa_handle* h = c.h;
   const bool graphs = h->cfg.cuda_graphs != 0 && a1 - a0 >= 3;
   for (int a = a0; a < (graphs ? a0 + 1 : a1); ++a) {
-    template_spectra_at(c, r.angles[a]);
     r.args.angle = a;
     r.args.angle_state = nullptr;
-    r.pairs += correlate_all(c, epi, h->ispec.as<float2>(), r.W, h->tspec.as<void>(), h->nt, r.args, r.D, r.E);
+    r.pairs += one_angle(c, r, epi, r.angles[a], nullptr);
   }
   if (!graphs) return;
   AngleState* table = buf<AngleState>(h->angle_table, r.angles.size());
@@ -893,7 +995,14 @@ void run_angles(Ctx& c, NormRun& r, int epi, int a0, int a1) {
 void norm_sweep1(Ctx& c, NormRun& r, int a0, int a1) {
   // with pruning the sums come with each pixel's best correlation (the same sums, added in the
   // same order)
-  run_angles(c, r, r.topk ? EPI_TOPK : r.prune ? EPI_SUMMAX : EPI_SUM, a0, a1);
+  const int epi = r.topk ? EPI_TOPK : r.prune ? EPI_SUMMAX : EPI_SUM;
+  const bool paired = sweep_paired(c.h->cfg, c.l, epi) && a1 > a0;
+  if (paired) {
+    const size_t bytes = pair_sum_bytes(c.l);
+    GISSPA_CUDA(cudaMemsetAsync(c.h->tsum.ensure(bytes), 0, bytes, c.s));
+  }
+  run_angles(c, r, epi, a0, a1);
+  if (paired) pair_sums(c, r.W, r.args.S1);
   r.phase = 2;
 }
 
@@ -912,7 +1021,7 @@ void norm_stats(Ctx& c, NormRun& r) {
     GISSPA_CUDA(cudaMemsetAsync(alive + rows, 0, r.W, c.s));
     GISSPA_CUDA(cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned), c.s));
     GISSPA_CUDA(cudaMemsetAsync(cnt + 2, 0xFF, sizeof(unsigned) * r.W, c.s));
-    row_alive_kernel<<<ceil_div(rows * 32, 256), 256, 0, c.s>>>(r.args.peak, ms, c.l, rows, r.args.thresh, alive,
+    row_alive_kernel<<<ceil_div(rows * 32, 256), 256, 0, c.s>>>(r.args.peak32, ms, c.l, rows, r.args.thresh, alive,
                                                                alive + rows, cnt, cnt + 2);
     GISSPA_LAUNCH_CHECK();
     pair_alive_kernel<<<ceil_div(npairs, 256), 256, 0, c.s>>>(r.args.pair_max, cnt + 2, r.W, r.n_angles, npairs,
@@ -1112,8 +1221,8 @@ void search_norm(Ctx& c, const float* d_img, int nx, int ny, std::vector<gisspa_
   norm_prepare(c, d_img, nx, ny, r);
   r.prune = h->cfg.prune_sweep2 != 0 && !r.topk && correlate_fast(c.l);
   if (r.prune) {  // sweep 1 keeps each pixel's best correlation and each pair's maximum
-    r.args.peak = buf<unsigned long long>(h->peak, r.npix);
-    GISSPA_CUDA(cudaMemsetAsync(r.args.peak, 0, sizeof(unsigned long long) * r.npix, c.s));
+    r.args.peak32 = buf<unsigned>(h->peak32, r.npix);
+    GISSPA_CUDA(cudaMemsetAsync(r.args.peak32, 0, sizeof(unsigned) * r.npix, c.s));
     r.n_angles = (int)r.angles.size();
     const size_t npairs = (size_t)r.W * r.n_angles * h->nt;
     r.args.pair_max = buf<unsigned>(h->pair_max, npairs);

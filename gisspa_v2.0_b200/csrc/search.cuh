@@ -80,12 +80,15 @@ struct gisspa_handle {
   // shells, statistics
   gisspa::DevBuf ra, rb, stats, scratch;
   // per-window-pixel state
-  gisspa::DevBuf S1, S2, peak, musig;
+  gisspa::DevBuf S1, S2, peak, peak32, musig;
   // correlation intermediate and outputs
   gisspa::DevBuf Q, cand, cand_count, nn_key, nn_sum, zkey, zcand, zcount;
   gisspa::DevBuf alive, alive_count, pair_max;  // rows and pairs sweep 2 transforms (prune_sweep2)
   gisspa::DevBuf prep_sub, tspec_sub, list_dev;  // the live templates of an angle of that sweep
   gisspa::DevBuf engine_ctr;  // work counters of the pair engine, one block per launch of a sequence
+  // paired sweep 1: template pairs' spectra of an angle, the running sum of all templates' spectra,
+  // that sum as one FP32 half spectrum, and its correlation maps
+  gisspa::DevBuf tpair, tsum, tsum_spec, sum_map;
   gisspa::DevBuf gen_z, gen_x;  // workspace of the generic correlation (window sizes without tuned kernels)
   gisspa::DevBuf dev_err;  // set by kernels whose bounded waits gave up
   // adjoint: whitened template spectra before weighting, RMS factors, dW/dpsi tables,
