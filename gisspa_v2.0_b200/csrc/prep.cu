@@ -252,62 +252,6 @@ __global__ void to_complex_kernel(const float* __restrict__ in, float2* __restri
   if (i < n) out[i] = make_float2(in[i], 0.f);
 }
 
-// LoadImage mean/sigma exactly as the reference's serial FP32 loop (norm.cu:157-167):
-// warps 1.. compute the per-element terms of the next tile while lane 0 of warp 0
-// accumulates the current tile in the original order.  IEEE intrinsics keep the
-// compiler from contracting or reordering.
-constexpr int kStatTile = 2048;
-__global__ void __launch_bounds__(1024) stats_serial_kernel(const float* __restrict__ img, long long n, float fnx,
-                                                            float fny, float* __restrict__ stats) {
-  __shared__ float t1[2][kStatTile], t2[2][kStatTile];
-  float sum = 0.f, sum_s2 = 0.f;
-  const long long ntiles = (n + kStatTile - 1) / kStatTile;
-  const int w = threadIdx.x >> 5;
-  // prologue: fill tile 0
-  for (int i = threadIdx.x; i < kStatTile; i += blockDim.x) {
-    if (i < n) {
-      const float cur = img[i];
-      t1[0][i] = __fdiv_rn(__fdiv_rn(cur, fnx), fny);
-      t2[0][i] = __fdiv_rn(__fdiv_rn(__fmul_rn(cur, cur), fnx), fny);
-    }
-  }
-  __syncthreads();
-  for (long long tI = 0; tI < ntiles; ++tI) {
-    const int cb = (int)(tI & 1);
-    if (w == 0) {
-      if (threadIdx.x == 0) {
-        const long long base = tI * kStatTile;
-        const int cnt = (int)min((long long)kStatTile, n - base);
-        for (int i = 0; i < cnt; ++i) {
-          sum = __fadd_rn(sum, t1[cb][i]);
-          sum_s2 = __fadd_rn(sum_s2, t2[cb][i]);
-        }
-      }
-    } else if (tI + 1 < ntiles) {
-      const long long base = (tI + 1) * kStatTile;
-      for (int i = threadIdx.x - 32; i < kStatTile; i += blockDim.x - 32) {
-        if (base + i < n) {
-          const float cur = img[base + i];
-          t1[cb ^ 1][i] = __fdiv_rn(__fdiv_rn(cur, fnx), fny);
-          t2[cb ^ 1][i] = __fdiv_rn(__fdiv_rn(__fmul_rn(cur, cur), fnx), fny);
-        }
-      }
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    const float avg = sum;
-    const float var = __fsqrt_rn(__fsub_rn(sum_s2, __fmul_rn(avg, avg)));
-    const float up = __fadd_rn(avg, __fmul_rn(6.f, var));
-    const float lo = __fsub_rn(avg, __fmul_rn(6.f, var));
-    stats[0] = avg;
-    stats[1] = (float)(int)up;  // int truncation (norm.cu:166-167)
-    stats[2] = (float)(int)lo;
-    stats[3] = (sum_s2 > __fmul_rn(avg, avg)) ? 1.f : 0.f;
-    if (!(up == up) || !(lo == lo)) stats[3] = 0.f;
-  }
-}
-
 __global__ void stats_fp64_kernel(const float* __restrict__ img, long long n, double* __restrict__ acc) {
   __shared__ double sh[32];
   double s = 0, s2 = 0;
@@ -527,18 +471,20 @@ void to_complex(const float* in, float2* out, long long n, cudaStream_t s) {
   GISSPA_LAUNCH_CHECK();
 }
 
-void image_stats(const float* img, int nx, int ny, bool fp32_serial, float* stats, double* scratch, cudaStream_t s) {
+size_t image_stats_bytes(int nx, int ny) { return serial_stats_bytes((long long)nx * ny); }
+
+void image_stats(const float* img, int nx, int ny, bool fp32_serial, float* stats, void* scratch, cudaStream_t s) {
   const long long n = (long long)nx * ny;
   if (fp32_serial) {
-    stats_serial_kernel<<<1, 1024, 0, s>>>(img, n, (float)nx, (float)ny, stats);
-    GISSPA_LAUNCH_CHECK();
-  } else {
-    GISSPA_CUDA(cudaMemsetAsync(scratch, 0, 2 * sizeof(double), s));
-    stats_fp64_kernel<<<std::min(ceil_div(n, kT), 1184), kT, 0, s>>>(img, n, scratch);
-    GISSPA_LAUNCH_CHECK();
-    stats_fp64_finish<<<1, 1, 0, s>>>(scratch, n, stats);
-    GISSPA_LAUNCH_CHECK();
+    serial_stats(img, nx, ny, stats, scratch, s);
+    return;
   }
+  double* acc = static_cast<double*>(scratch);
+  GISSPA_CUDA(cudaMemsetAsync(acc, 0, 2 * sizeof(double), s));
+  stats_fp64_kernel<<<std::min(ceil_div(n, kT), 1184), kT, 0, s>>>(img, n, acc);
+  GISSPA_LAUNCH_CHECK();
+  stats_fp64_finish<<<1, 1, 0, s>>>(acc, n, stats);
+  GISSPA_LAUNCH_CHECK();
 }
 
 void image_load(const float* img, long long n, const float* stats, bool clamp, bool invert, float2* out, cudaStream_t s) {

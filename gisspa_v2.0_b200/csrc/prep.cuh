@@ -33,8 +33,12 @@ void real_part(const float2* in, float* out, long long n, float scale, cudaStrea
 void to_complex(const float* in, float2* out, long long n, cudaStream_t s);
 
 // ---- micrograph
-// LoadImage statistics (norm.cu:157-167): stats = {avg, up_bound, low_bound, clamp}
-void image_stats(const float* img, int nx, int ny, bool fp32_serial, float* stats, double* scratch, cudaStream_t s);
+// LoadImage statistics (norm.cu:157-167): stats = {avg, up_bound, low_bound, clamp}; fp32_serial:
+// the reference's running FP32 sums, bit for bit (serial_sum.cu).  scratch: image_stats_bytes.
+size_t image_stats_bytes(int nx, int ny);
+void image_stats(const float* img, int nx, int ny, bool fp32_serial, float* stats, void* scratch, cudaStream_t s);
+size_t serial_stats_bytes(long long n);
+void serial_stats(const float* img, int nx, int ny, float* stats, void* scratch, cudaStream_t s);
 // clamp (norm) + invert, to complex
 void image_load(const float* img, long long n, const float* stats, bool clamp, bool invert, float2* out,
                 cudaStream_t s);

@@ -791,8 +791,7 @@ void norm_prepare(Ctx& c, const float* d_img, int nx, int ny, NormRun& r) {
   r.ny = ny;
   r.N = (long long)nx * ny;
   GISSPA_CUDA(cudaEventRecord(h->ev[0], c.s));
-  // LoadImage statistics on the side stream (the serial FP32 form occupies one SM for
-  // ~4 ns per pixel) while the templates are prepared on the main stream
+  // LoadImage statistics on the side stream while the templates are prepared on the main stream
   const bool prefetched = h->next_dev == d_img && h->next_nx == nx && h->next_ny == ny;
   h->next_dev = nullptr;
   if (prefetched) {
@@ -801,7 +800,7 @@ void norm_prepare(Ctx& c, const float* d_img, int nx, int ny, NormRun& r) {
     h->scratch.swap(h->scratch_next);
   } else {
     float* st0 = buf<float>(h->stats, 4);
-    double* scr = buf<double>(h->scratch, 16);
+    void* scr = h->scratch.ensure(image_stats_bytes(nx, ny));
     GISSPA_CUDA(cudaEventRecord(h->ev_in, c.s));
     GISSPA_CUDA(cudaStreamWaitEvent(h->side, h->ev_in, 0));
     image_stats(d_img, nx, ny, (cfg.quirks & GISSPA_QUIRK_OUTLIER_FP32_SERIAL) != 0, st0, scr, h->side);
@@ -1497,7 +1496,7 @@ void debug_stage(gisspa_handle* h, int what, const float* d_img, int nx, int ny,
   if (!d_img) throw CudaError{cudaErrorInvalidValue, "debug_stage: image required"};
   const long long N = (long long)nx * ny;
   float* stats = buf<float>(h->stats, 4);
-  double* scr = buf<double>(h->scratch, 16);
+  void* scr = h->scratch.ensure(image_stats_bytes(nx, ny));
   image_stats(d_img, nx, ny, (cfg.quirks & GISSPA_QUIRK_OUTLIER_FP32_SERIAL) != 0, stats, scr, c.s);
   float2* G = buf<float2>(h->img_c, N);
   image_load(d_img, N, stats, true, cfg.invert != 0, G, c.s);
@@ -1926,7 +1925,7 @@ int run_batch(gisspa_handle* h, int n, const float* const* images, const int* nx
   h->next_dev = nullptr;
   // Micrographs alternate between two device buffers.  While micrograph i's first sweep runs
   // (norm_type=1), the host uploads micrograph i+1 into the other buffer on the side stream and
-  // queues its LoadImage statistics (one thread, ~65 ms at 4096^2) there; search i+1 then starts
+  // queues its LoadImage statistics there; search i+1 then starts
   // from them.  Buffer i+1 last held micrograph i-1, whose search has returned.
   gisspa::DevBuf* bufs[2] = {&h->img_in, &h->img_next};
   for (int i = 0; i < n; ++i) {
@@ -1946,7 +1945,7 @@ int run_batch(gisspa_handle* h, int n, const float* const* images, const int* nx
           const size_t b2 = sizeof(float) * (size_t)nx[i + 1] * ny[i + 1];
           float* dst = static_cast<float*>(nb.ensure(b2));
           float* st1 = buf<float>(h->stats_next, 4);
-          double* scr = buf<double>(h->scratch_next, 16);
+          void* scr = h->scratch_next.ensure(image_stats_bytes(nx[i + 1], ny[i + 1]));
           GISSPA_CUDA(cudaMemcpyAsync(dst, images[i + 1], b2, cudaMemcpyHostToDevice, h->side));
           image_stats(dst, nx[i + 1], ny[i + 1], (h->cfg.quirks & GISSPA_QUIRK_OUTLIER_FP32_SERIAL) != 0, st1, scr,
                       h->side);
