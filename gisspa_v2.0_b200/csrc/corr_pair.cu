@@ -72,6 +72,11 @@ __device__ __forceinline__ void team_sync(int team) {
     asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(T) : "memory");
 }
 
+// Writes v into the low or high half of w.
+__device__ __forceinline__ void put_half(unsigned& w, int high, int v) {
+  w = high ? (w & 0xFFFFu) | (unsigned)v << 16 : (w & 0xFFFF0000u) | (unsigned)v;
+}
+
 // Column pass: NC columns kx (and their mirror images -kx) per CTA, one (window, template pair)
 // per blockIdx.y.  Stage 1: L / R1 threads per column, R1 points each, the loads coalesced
 // along ky.  One exchange, then stage 2's butterflies are dealt over the CTA with the column as
@@ -277,14 +282,13 @@ __global__ void __launch_bounds__(2 * RowPlan2<L>::T* RB* DS, MINB)
           m2 = fmaxf(m2, cm);
         }
         if constexpr (TOPK) {
-          constexpr unsigned keep = 0xFFFF0000u;
           if (c1 > best[i]) {
             best[i] = c1;
-            barg[i / 2] = i & 1 ? (barg[i / 2] & ~keep) | (unsigned)(d + 1) << 16 : (barg[i / 2] & keep) | (unsigned)(d + 1);
+            put_half(barg[i / 2], i & 1, d + 1);
           }
           if (two && c2 > best[i]) {
             best[i] = c2;
-            barg[i / 2] = i & 1 ? (barg[i / 2] & ~keep) | (unsigned)(d + 2) << 16 : (barg[i / 2] & keep) | (unsigned)(d + 2);
+            put_half(barg[i / 2], i & 1, d + 2);
           }
         }
       }
@@ -334,7 +338,7 @@ __global__ void __launch_bounds__(2 * RowPlan2<L>::T* RB* DS, MINB)
           const unsigned g = i & 1 ? g2 >> 16 : g2 & 0xFFFFu, own = i & 1 ? barg[i / 2] >> 16 : barg[i / 2] & 0xFFFFu;
           if (g && (b > best[i] || (b == best[i] && g < own))) {
             best[i] = b;
-            barg[i / 2] = i & 1 ? (barg[i / 2] & 0xFFFFu) | g << 16 : (barg[i / 2] & 0xFFFF0000u) | g;
+            put_half(barg[i / 2], i & 1, (int)g);
           }
         }
       }
@@ -362,7 +366,9 @@ __global__ void __launch_bounds__(2 * RowPlan2<L>::T* RB* DS, MINB)
       const unsigned key = float_key(best[i] * inv);
       if constexpr (TOPK) {
         const unsigned g = i & 1 ? barg[i / 2] >> 16 : barg[i / 2] & 0xFFFFu;
-        if (g) atomicMax(a.peak + pix, (unsigned long long)key << 32 | (unsigned)(0xFFFFFFFFu - (unsigned)(id0 + (int)g)));
+        if (g)
+          atomicMax(a.peak + pix,
+                    (unsigned long long)key << 32 | (unsigned)(0xFFFFFFFFu - (unsigned)(id0 + (int)g)));
       } else {
         atomicMax(a.peak32 + pix, key);
       }

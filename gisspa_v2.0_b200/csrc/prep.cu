@@ -334,6 +334,22 @@ __global__ void gather_windows_kernel(const float* __restrict__ img, int nx, int
   out[(size_t)b * l * l + k] = make_float2(v, 0.f);
 }
 
+// Bilinear sample of the image rotated by (cose, sine) at pixel id (rotate_subIMG,
+// kernels.cu:545-579, with its float expressions).
+__device__ __forceinline__ float rotated_sample(const float* __restrict__ src, int l, int id, float cose, float sine) {
+  const int i = id % l, j = id / l;
+  const float x = (float)(i - l / 2), y = (float)(j - l / 2);
+  const float x2 = (cose * x + sine * y) + l / 2;
+  const float y2 = (-sine * x + cose * y) + l / 2;
+  if (x2 < 0 || x2 > l - 1.0f || y2 < 0 || y2 > l - 1.0f) return 0.f;
+  const int ii = (int)floorf(x2), jj = (int)floorf(y2);
+  int k0 = ii + jj * l, k1 = k0 + 1, k2 = k0 + l + 1, k3 = k0 + l;
+  if (ii == l - 1) { k1 -= 1; k2 -= 1; }
+  if (jj == l - 1) { k2 -= l; k3 -= l; }
+  const float t = x2 - ii, u = y2 - jj, tt = 1.0f - t, uu = 1.0f - u;
+  return src[k0] * tt * uu + src[k1] * t * uu + src[k2] * t * u + src[k3] * tt * u;
+}
+
 __global__ void rotate_kernel(const float* __restrict__ in, int l, float cose, float sine, int mask, float d_m,
                               float ehw, float2* __restrict__ out, double* __restrict__ sums,
                               const AngleState* __restrict__ st) {
@@ -347,20 +363,9 @@ __global__ void rotate_kernel(const float* __restrict__ in, int l, float cose, f
   const float* src = in + (size_t)n * l * l;
   float res = 0.f;
   if (id < l * l) {
-    const int i = id % l, j = id / l;
-    const float x = (float)(i - l / 2), y = (float)(j - l / 2);
-    // same float expression as rotate_subIMG (kernels.cu:554-555)
-    const float x2 = (cose * x + sine * y) + l / 2;
-    const float y2 = (-sine * x + cose * y) + l / 2;
-    if (!(x2 < 0 || x2 > l - 1.0f || y2 < 0 || y2 > l - 1.0f)) {
-      const int ii = (int)floorf(x2), jj = (int)floorf(y2);
-      int k0 = ii + jj * l, k1 = k0 + 1, k2 = k0 + l + 1, k3 = k0 + l;
-      if (ii == l - 1) { k1 -= 1; k2 -= 1; }
-      if (jj == l - 1) { k2 -= l; k3 -= l; }
-      const float t = x2 - ii, u = y2 - jj, tt = 1.0f - t, uu = 1.0f - u;
-      res = src[k0] * tt * uu + src[k1] * t * uu + src[k2] * t * u + src[k3] * tt * u;
-    }
+    res = rotated_sample(src, l, id, cose, sine);
     if (mask) {
+      const int i = id % l, j = id / l;
       const float dm = 1.5f * d_m;
       const float r = hypotf((float)(i - l / 2), (float)(j - l / 2));
       if (r > dm / 2 + 2 * ehw) res = 0.f;
@@ -376,6 +381,16 @@ __global__ void rotate_kernel(const float* __restrict__ in, int l, float cose, f
       atomicAdd(sums + 2 * n + 1, s2);
     }
   }
+}
+
+// The norm_type=0 search rotates the windows instead of the templates: image b = a W + w of the
+// output is window w rotated by angle a of the table (the samples of rotate_kernel, no mask).
+__global__ void rotate_windows_kernel(const float* __restrict__ in, int W, int l, const AngleState* __restrict__ table,
+                                      float2* __restrict__ out) {
+  const int b = blockIdx.y, id = blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= l * l) return;
+  const float cose = table[b / W].cose, sine = table[b / W].sine;
+  out[(size_t)b * l * l + id] = make_float2(rotated_sample(in + (size_t)(b % W) * l * l, l, id, cose, sine), 0.f);
 }
 
 template <typename SPEC>
@@ -514,6 +529,11 @@ void rotate_batch(const float* in, int n, int l, float cose, float sine, bool ma
   if (sums) GISSPA_CUDA(cudaMemsetAsync(sums, 0, sizeof(double) * 2 * n, s));
   rotate_kernel<<<dim3(ceil_div((long long)l * l, kT), n), kT, 0, s>>>(in, l, cose, sine, mask ? 1 : 0, d_m, ehw, out,
                                                                        sums, st);
+  GISSPA_LAUNCH_CHECK();
+}
+
+void rotate_windows(const float* in, int W, int A, int l, const AngleState* table, float2* out, cudaStream_t s) {
+  rotate_windows_kernel<<<dim3(ceil_div((long long)l * l, kT), W * A), kT, 0, s>>>(in, W, l, table, out);
   GISSPA_LAUNCH_CHECK();
 }
 

@@ -1316,15 +1316,27 @@ void search_nonorm(Ctx& c, const float* d_img, int nx, int ny, std::vector<gissp
   std::vector<int> woff(bx);
   for (int k = 0; k < bx; ++k) woff[k] = k * (l - cfg.overlap);  // split_IMG unclamped (kernels.cu:605-624)
   const std::vector<float> angles = angle_list(cfg.phistep);
-  int D, E;
-  choose_batches(cfg, l, W, nt, D, E);
   const long long TS2 = (long long)ts * ts;
   int* dtx = buf<int>(h->offx, std::max<size_t>(woff.size(), 2));
   int* dty = buf<int>(h->offy, std::max<size_t>(woff.size(), 2));
-  unsigned long long* nk = buf<unsigned long long>(h->nn_key, (size_t)W * nt);
-  double* nsum = buf<double>(h->nn_sum, (size_t)W * nt * 2);
-  std::vector<unsigned long long> hk((size_t)W * nt);
-  std::vector<double> hsum((size_t)W * nt * 2);
+  // Several angles go through each launch: rotated windows a W + w are so many more windows to
+  // the correlation.  One angle of a 720^2 tile is 4 windows, 32 correlations with 8 templates: too
+  // few to fill the GPU, and its dozen launches, copies and the host's merge cost 140 us each.  At
+  // most 256 MB of rotated windows (128 of 512^2).
+  const long long most = std::max(1LL, (256LL << 20) / (W * c.L2 * (long long)sizeof(float2)));
+  const int groups = (int)(((long long)angles.size() + most - 1) / most);
+  const int AB = ((int)angles.size() + groups - 1) / groups;
+  unsigned long long* nk = buf<unsigned long long>(h->nn_key, (size_t)AB * W * nt);
+  double* nsum = buf<double>(h->nn_sum, (size_t)AB * W * nt * 2);
+  std::vector<unsigned long long> hk((size_t)AB * W * nt);
+  std::vector<double> hsum((size_t)AB * W * nt * 2);
+  std::vector<AngleState> table(angles.size());
+  for (size_t a = 0; a < table.size(); ++a) {
+    const double rad = (double)angles[a] * kRefPi / 180.0;
+    table[a] = AngleState{(int)a, (float)std::cos(rad), (float)std::sin(rad), 0};
+  }
+  AngleState* dtable = buf<AngleState>(h->angle_table, table.size());
+  GISSPA_CUDA(cudaMemcpyAsync(dtable, table.data(), sizeof(AngleState) * table.size(), cudaMemcpyHostToDevice, c.s));
   long long pairs = 0;
   // top-K: every (tile, angle, window) peak of each template that passes the reference's
   // centre test and the threshold, in that generation order
@@ -1360,89 +1372,92 @@ void search_nonorm(Ctx& c, const float* d_img, int nx, int ny, std::vector<gissp
     }
     float* wr = buf<float>(h->win_real, (size_t)W * c.L2);
     real_part(w, wr, (long long)W * c.L2, 1.f, c.s);
-    for (size_t a = 0; a < angles.size(); ++a) {
-      const float e = angles[a];
-      const double rad = (double)e * kRefPi / 180.0;
+    for (size_t a0 = 0; a0 < angles.size(); a0 += AB) {
+      const int na = (int)std::min<size_t>(AB, angles.size() - a0), WA = na * W;
       // PickParticles (nonorm.cu:452-537): rotate the windows, transform, correlate
-      float2* rot = buf<float2>(h->rot, (size_t)W * c.L2);
-      float2* rtmp = buf<float2>(h->rot_tmp, (size_t)W * hs * l);
-      rotate_batch(wr, W, l, (float)std::cos(rad), (float)std::sin(rad), false, 0.f, 0.f, rot, nullptr, c.s);
-      h->fft.rows(rot, (long long)W * l, l, -1, 1.f, c.s);
-      h->fft.transpose(rot, rtmp, W, l, l, c.s, hs);
-      h->fft.rows(rtmp, (long long)W * hs, l, -1, 1.f, c.s);
-      float2* I = buf<float2>(h->ispec, (size_t)W * hs * l);
-      finalize_spectra(rtmp, W, l, nullptr, GISSPA_SPEC_FP32, I, 1.0 / (double)c.L2, c.s);
-      GISSPA_CUDA(cudaMemsetAsync(nk, 0, sizeof(unsigned long long) * W * nt, c.s));
-      GISSPA_CUDA(cudaMemsetAsync(nsum, 0, sizeof(double) * W * nt * 2, c.s));
+      float2* rot = buf<float2>(h->rot, (size_t)AB * W * c.L2);
+      float2* I = buf<float2>(h->ispec, (size_t)AB * W * hs * l);
+      rotate_windows(wr, W, na, l, dtable + a0, rot, c.s);
+      h->fft.rows(rot, (long long)WA * l, l, -1, 1.f, c.s);
+      h->fft.transpose(rot, I, WA, l, l, c.s, hs);
+      h->fft.rows(I, (long long)WA * hs, l, -1, (float)(1.0 / (double)c.L2), c.s);
+      GISSPA_CUDA(cudaMemsetAsync(nk, 0, sizeof(unsigned long long) * WA * nt, c.s));
+      GISSPA_CUDA(cudaMemsetAsync(nsum, 0, sizeof(double) * WA * nt * 2, c.s));
       CorrArgs args{};
       args.nt_real = nt;
       args.nt_total = nt;
-      args.angle = (int)a;
       args.nn_key = nk;
       args.nn_sum = nsum;
       args.border = cfg.diameter / 4;
-      pairs += correlate_all(c, EPI_NONORM, I, W, h->tspec.as<void>(), nt, args, D, E);
-      GISSPA_CUDA(cudaMemcpyAsync(hk.data(), nk, sizeof(unsigned long long) * W * nt, cudaMemcpyDeviceToHost, c.s));
-      GISSPA_CUDA(cudaMemcpyAsync(hsum.data(), nsum, sizeof(double) * W * nt * 2, cudaMemcpyDeviceToHost, c.s));
+      int D, E;
+      choose_batches(cfg, l, WA, nt, D, E);
+      pairs += correlate_all(c, EPI_NONORM, I, WA, h->tspec.as<void>(), nt, args, D, E);
+      GISSPA_CUDA(cudaMemcpyAsync(hk.data(), nk, sizeof(unsigned long long) * WA * nt, cudaMemcpyDeviceToHost, c.s));
+      GISSPA_CUDA(cudaMemcpyAsync(hsum.data(), nsum, sizeof(double) * WA * nt * 2, cudaMemcpyDeviceToHost, c.s));
       GISSPA_CUDA(cudaStreamSynchronize(c.s));
-      // host merge (nonorm.cu:498-534): best window per template, centre rotated back
-      std::vector<float> bs(nt, 0.f), bxp(nt, 0.f), byp(nt, 0.f);
-      const double ce = std::cos(rad), se = std::sin(rad);
-      for (int b = 0; b < W; ++b) {
-        const int i = b % bx, j = b / bx;
-        for (int n = 0; n < nt; ++n) {
-          const unsigned long long k = hk[(size_t)b * nt + n];
-          double peak = 0, pos = 0;
-          if (k) {
-            uint32_t hi = (uint32_t)(k >> 32);
-            uint32_t bits = (hi & 0x80000000u) ? (hi & 0x7fffffffu) : ~hi;
-            float pv;
-            std::memcpy(&pv, &bits, 4);
-            // low word: (0xFFFFF - chunk) << 8 | (255 - brev8(position in the chunk))
-            const unsigned lo = (unsigned)(k & 0xFFFFFFFFu);
-            const int chunk = (int)(0xFFFFFu - (lo >> 8));
-            unsigned t = 255u - (lo & 0xFFu), tb = 0;
-            for (int bit = 0; bit < 8; ++bit) tb |= ((t >> bit) & 1u) << (7 - bit);
-            peak = pv;
-            pos = (double)(chunk * 256 + (int)tb);
-          }
-          const double s1 = hsum[2 * ((size_t)b * nt + n)], s2 = hsum[2 * ((size_t)b * nt + n) + 1];
-          const double rA = s1 - peak, rB = s2 - peak * peak, rC = (double)c.L2 - 1;
-          const double sd = std::sqrt(rB / rC - (rA / rC) * (rA / rC));
-          const double score = sd == 0 ? 0.0 : peak / sd;
-          const int cx = (int)pos % l, cy = (int)pos / l;
-          const double centerx = i * (l - cfg.overlap) + (cx - l / 2) * ce + (cy - l / 2) * se + l / 2;
-          const double centery = j * (l - cfg.overlap) + (cy - l / 2) * ce - (cx - l / 2) * se + l / 2;
-          const bool valid = centerx >= 0 && centerx < ts && centery >= 0 && centery < ts;
-          if (topk) {
-            if (valid && (float)score >= cfg.threshold)
-              cands[n].push_back(NonormCand{score, (float)(tx[t] + centerx), (float)(ty[t] + centery), (int)t,
-                                            (int)a, b});
-            continue;
-          }
-          if (bs[n] < (float)score && valid) {
-            bs[n] = (float)score;
-            bxp[n] = (float)centerx;
-            byp[n] = (float)centery;
+      for (int ia = 0; ia < na; ++ia) {
+        const size_t a = a0 + ia, first = (size_t)ia * W * nt;  // this angle's (window, template) results
+        const float e = angles[a];
+        const double rad = (double)e * kRefPi / 180.0;
+        // host merge (nonorm.cu:498-534): best window per template, centre rotated back
+        std::vector<float> bs(nt, 0.f), bxp(nt, 0.f), byp(nt, 0.f);
+        const double ce = std::cos(rad), se = std::sin(rad);
+        for (int b = 0; b < W; ++b) {
+          const int i = b % bx, j = b / bx;
+          for (int n = 0; n < nt; ++n) {
+            const unsigned long long k = hk[first + (size_t)b * nt + n];
+            double peak = 0, pos = 0;
+            if (k) {
+              uint32_t hi = (uint32_t)(k >> 32);
+              uint32_t bits = (hi & 0x80000000u) ? (hi & 0x7fffffffu) : ~hi;
+              float pv;
+              std::memcpy(&pv, &bits, 4);
+              // low word: (0xFFFFF - chunk) << 8 | (255 - brev8(position in the chunk))
+              const unsigned lo = (unsigned)(k & 0xFFFFFFFFu);
+              const int chunk = (int)(0xFFFFFu - (lo >> 8));
+              unsigned t = 255u - (lo & 0xFFu), tb = 0;
+              for (int bit = 0; bit < 8; ++bit) tb |= ((t >> bit) & 1u) << (7 - bit);
+              peak = pv;
+              pos = (double)(chunk * 256 + (int)tb);
+            }
+            const double s1 = hsum[2 * (first + (size_t)b * nt + n)], s2 = hsum[2 * (first + (size_t)b * nt + n) + 1];
+            const double rA = s1 - peak, rB = s2 - peak * peak, rC = (double)c.L2 - 1;
+            const double sd = std::sqrt(rB / rC - (rA / rC) * (rA / rC));
+            const double score = sd == 0 ? 0.0 : peak / sd;
+            const int cx = (int)pos % l, cy = (int)pos / l;
+            const double centerx = i * (l - cfg.overlap) + (cx - l / 2) * ce + (cy - l / 2) * se + l / 2;
+            const double centery = j * (l - cfg.overlap) + (cy - l / 2) * ce - (cx - l / 2) * se + l / 2;
+            const bool valid = centerx >= 0 && centerx < ts && centery >= 0 && centery < ts;
+            if (topk) {
+              if (valid && (float)score >= cfg.threshold)
+                cands[n].push_back(NonormCand{score, (float)(tx[t] + centerx), (float)(ty[t] + centery), (int)t,
+                                              (int)a, b});
+              continue;
+            }
+            if (bs[n] < (float)score && valid) {
+              bs[n] = (float)score;
+              bxp[n] = (float)centerx;
+              byp[n] = (float)centery;
+            }
           }
         }
+        if (topk) continue;
+        for (int n = 0; n < nt; ++n)  // OutputScore (nonorm.cu:539-557)
+          if (bs[n] >= cfg.threshold) {
+            gisspa_pick pk{};
+            pk.score = bs[n];
+            pk.x = bxp[n];
+            pk.y = byp[n];
+            pk.angle = e;
+            pk.theta = e;
+            pk.template_id = n;
+            pk.window = -1;
+            pk.tile = (int)t;
+            pk.angle_index = (int)a;
+            pk.chunk = -1;
+            out.push_back(pk);
+          }
       }
-      if (topk) continue;
-      for (int n = 0; n < nt; ++n)  // OutputScore (nonorm.cu:539-557)
-        if (bs[n] >= cfg.threshold) {
-          gisspa_pick pk{};
-          pk.score = bs[n];
-          pk.x = bxp[n];
-          pk.y = byp[n];
-          pk.angle = e;
-          pk.theta = e;
-          pk.template_id = n;
-          pk.window = -1;
-          pk.tile = (int)t;
-          pk.angle_index = (int)a;
-          pk.chunk = -1;
-          out.push_back(pk);
-        }
     }
   }
   GISSPA_CUDA(cudaEventRecord(h->ev[2], c.s));
