@@ -23,45 +23,10 @@
 #include "../../include/gisspa.h"
 #include "correlate.cuh"
 #include "fft_pair.cuh"
+#include "pair_spec.cuh"
 
 namespace gisspa {
 namespace {
-
-// A template pair's spectra at one point, as the column pass reads them.  FP32: U = T1 - i T2
-// and V = T1 + i T2 (so that I conj U = A1 + i A2 and I conj V = A1 - i A2) as
-// (U.re, V.re, U.im, V.im).  FP16 / BF16: T1 and T2 themselves, rounded as the one-template
-// form rounds them.
-struct PairFp32 {
-  using T = float4;
-  __device__ __forceinline__ static float2 plus(float2 i, T t) { return cmulc(i, make_float2(t.x, t.z)); }
-  __device__ __forceinline__ static Cx2 both(float2 i, T t) {
-    const float2 a = cmulc(i, make_float2(t.x, t.z)), b = cmulc(i, make_float2(t.y, t.w));
-    return Cx2{make_float2(a.x, b.x), make_float2(a.y, b.y)};
-  }
-  __device__ __forceinline__ static float2 round(float2 t) { return t; }
-  __device__ __forceinline__ static T pack(float2 t1, float2 t2) {
-    return make_float4(t1.x + t2.y, t1.x - t2.y, t1.y - t2.x, t1.y + t2.x);
-  }
-};
-template <typename SPEC>
-struct PairHalf {
-  struct __align__(8) T {
-    typename SPEC::T t1, t2;
-  };
-  __device__ __forceinline__ static Cx2 both(float2 i, T t) {
-    const float2 a1 = cmulc(i, SPEC::load(&t.t1)), a2 = cmulc(i, SPEC::load(&t.t2));
-    return Cx2{make_float2(a1.x - a2.y, a1.x + a2.y), make_float2(a1.y + a2.x, a1.y - a2.x)};
-  }
-  __device__ __forceinline__ static float2 plus(float2 i, T t) {
-    const Cx2 c = both(i, t);
-    return make_float2(c.re.x, c.im.x);
-  }
-  __device__ __forceinline__ static float2 round(float2 t) {
-    const typename SPEC::T r = SPEC::pack(t);
-    return SPEC::load(&r);
-  }
-  __device__ __forceinline__ static T pack(float2 t1, float2 t2) { return T{SPEC::pack(t1), SPEC::pack(t2)}; }
-};
 
 // Barrier of a team: a warp or half warp, or whole warps through named barrier 1 + team.
 template <int T>
@@ -348,8 +313,10 @@ __global__ void __launch_bounds__(2 * RowPlan2<L>::T* RB* DS, MINB)
   }
   if constexpr (MAXP) {
     if (a.pair_max)
-      for (int d = threadIdx.x; d < a.D; d += RB * TT)
-        atomicMax(a.pair_max + pair_index(win, a.n0 + d, angle, a.n_windows, a.n_angles), pmax[d]);
+      for (int d = threadIdx.x; d < a.D; d += RB * TT) {
+        const int v = a.n0 + d, da = v / a.nt_real;  // image v: template v % nt at the da-th angle
+        atomicMax(a.pair_max + pair_index(win, v - da * a.nt_real, angle + da, a.n_windows, a.n_angles), pmax[d]);
+      }
   }
   // Fold into the per-pixel state with reductions that return nothing (no warp waits on the
   // state's memory latency); each pixel receives one per launch and launches are
@@ -376,47 +343,49 @@ __global__ void __launch_bounds__(2 * RowPlan2<L>::T* RB* DS, MINB)
   }
 }
 
-// Half spectra X[n][kx][ky] of single templates -> the column pass's pairs, scaled and with DC
-// zeroed as finalize_spectra (prep.cu) does; an odd last template is paired with zeros.  The
-// values as stored (rounded to FP16 / BF16 there) are also added up over the templates, in FP64,
-// one slot of tsum per blockIdx.y: the sum of the correlations over all templates and angles is
-// the correlation with the sum of the templates (pair_sum_finish).
-constexpr int kSumSlots = 8;
+// Half spectra X[n][kx][ky] of single templates -> pairs, scaled and with DC zeroed as
+// finalize_spectra (prep.cu) does; an odd last template is paired with zeros.
 template <typename SPEC>
-__global__ void __launch_bounds__(256) pair_spectra_kernel(const float2* __restrict__ X, int nt, int l,
-                                                           const double* __restrict__ sums,
-                                                           typename SPEC::T* __restrict__ out, double base,
-                                                           double2* __restrict__ tsum) {
-  extern __shared__ float fs[];  // [2 np]: this block's templates
-  const int np_all = (nt + 1) / 2, per_y = (np_all + gridDim.y - 1) / gridDim.y;
-  const int g0 = blockIdx.y * per_y, g1 = min(np_all, g0 + per_y);
+__global__ void __launch_bounds__(256) pair_pack_kernel(const float2* __restrict__ X, int n, int l,
+                                                        const double* __restrict__ sums,
+                                                        typename SPEC::T* __restrict__ out, double base) {
+  const int g = blockIdx.y;
+  const bool two = 2 * g + 1 < n;
   const long long per = (long long)(l / 2 + 1) * l;
   const double L2 = (double)l * l;
-  for (int j = threadIdx.x; j < 2 * (g1 - g0); j += blockDim.x) {
-    const int n = 2 * g0 + j;
-    float f = 0.f;
-    if (n < nt) {
-      const double mean = sums[2 * n] / L2, var = sums[2 * n + 1] / L2 - mean * mean;
-      f = (float)(var != 0 ? base / sqrt(var) : base);
-    }
-    fs[j] = f;
+  float fs[2] = {0.f, 0.f};
+  for (int j = 0; j < (two ? 2 : 1); ++j) {
+    const int i = 2 * g + j;
+    const double mean = sums[2 * i] / L2, var = sums[2 * i + 1] / L2 - mean * mean;
+    fs[j] = (float)(var != 0 ? base / sqrt(var) : base);
   }
-  __syncthreads();
+  const float2* X1 = X + (size_t)2 * g * per;
+  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < per; k += (long long)gridDim.x * blockDim.x) {
+    float2 t1 = make_float2(0.f, 0.f), t2 = t1;
+    if (k) {  // mean subtracted: DC is exactly zero
+      t1 = cscale(X1[k], fs[0]);
+      if (two) t2 = cscale(X1[per + k], fs[1]);
+    }
+    out[(size_t)g * per + k] = SPEC::pack(t1, t2);
+  }
+}
+
+// Adds the spectra of all templates (as stored) to the running sum, in FP64, one slot of tsum per
+// blockIdx.y: the sum of the correlations over all templates and angles is the correlation with
+// the sum of the templates (pair_sum_finish).
+constexpr int kSumSlots = 8;
+template <typename SPEC>
+__global__ void __launch_bounds__(256) pair_sum_kernel(const typename SPEC::T* __restrict__ T, int np, long long per,
+                                                       double2* __restrict__ tsum) {
+  const int per_y = (np + gridDim.y - 1) / gridDim.y, g0 = blockIdx.y * per_y, g1 = min(np, g0 + per_y);
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= per) return;
   double2 acc = make_double2(0.0, 0.0);
-#pragma unroll 4
+#pragma unroll 8
   for (int g = g0; g < g1; ++g) {
-    float2 t1 = make_float2(0.f, 0.f), t2 = t1;
-    if (k) {  // mean subtracted: DC is exactly zero
-      t1 = cscale(X[(size_t)2 * g * per + k], fs[2 * (g - g0)]);
-      if (2 * g + 1 < nt) t2 = cscale(X[((size_t)2 * g + 1) * per + k], fs[2 * (g - g0) + 1]);
-    }
-    t1 = SPEC::round(t1);
-    t2 = SPEC::round(t2);
-    acc.x += (double)t1.x + (double)t2.x;
-    acc.y += (double)t1.y + (double)t2.y;
-    out[(size_t)g * per + k] = SPEC::pack(t1, t2);
+    const double2 v = SPEC::sum(T[(size_t)g * per + k]);
+    acc.x += v.x;
+    acc.y += v.y;
   }
   double2* o = tsum + (size_t)blockIdx.y * per + k;
   o->x += acc.x;
@@ -540,24 +509,35 @@ size_t pair_spectrum_bytes(int L, int spec) {
 
 size_t pair_sum_bytes(int L) { return sizeof(double2) * kSumSlots * (size_t)(L / 2 + 1) * L; }
 
-void pair_spectra(const float2* X, int nt, int L, const double* sums, int spec, void* out, double base, void* tsum,
-                  cudaStream_t s) {
+void pair_pack(const float2* X, int n, int L, const double* sums, int spec, void* out, double base, cudaStream_t s) {
+  const dim3 grid((unsigned)std::min(ceil_div((long long)(L / 2 + 1) * L, 1024), 512), (unsigned)((n + 1) / 2));
+  if (spec == GISSPA_SPEC_FP16)
+    pair_pack_kernel<PairHalf<SpecFp16>>
+        <<<grid, 256, 0, s>>>(X, n, L, sums, static_cast<PairHalf<SpecFp16>::T*>(out), base);
+  else if (spec == GISSPA_SPEC_BF16)
+    pair_pack_kernel<PairHalf<SpecBf16>>
+        <<<grid, 256, 0, s>>>(X, n, L, sums, static_cast<PairHalf<SpecBf16>::T*>(out), base);
+  else
+    throw CudaError{cudaErrorInvalidValue, "FP32 pairs come from tmpl_spectra"};
+  GISSPA_LAUNCH_CHECK();
+}
+
+void pair_sum(const void* T, int nt, int L, int spec, void* tsum, cudaStream_t s) {
   const long long per = (long long)(L / 2 + 1) * L;
-  const int np = (nt + 1) / 2, gy = std::min(kSumSlots, np);
-  const dim3 grid((unsigned)ceil_div(per, 256), (unsigned)gy);
-  const size_t smem = sizeof(float) * 2 * ((np + gy - 1) / gy);
+  const int np = (nt + 1) / 2;
+  const dim3 grid((unsigned)ceil_div(per, 256), (unsigned)std::min(kSumSlots, np));
   double2* ts = static_cast<double2*>(tsum);
   switch (spec) {
     case GISSPA_SPEC_FP32:
-      pair_spectra_kernel<PairFp32><<<grid, 256, smem, s>>>(X, nt, L, sums, static_cast<float4*>(out), base, ts);
+      pair_sum_kernel<PairFp32><<<grid, 256, 0, s>>>(static_cast<const PairFp32::T*>(T), np, per, ts);
       break;
     case GISSPA_SPEC_FP16:
-      pair_spectra_kernel<PairHalf<SpecFp16>>
-          <<<grid, 256, smem, s>>>(X, nt, L, sums, static_cast<PairHalf<SpecFp16>::T*>(out), base, ts);
+      pair_sum_kernel<PairHalf<SpecFp16>>
+          <<<grid, 256, 0, s>>>(static_cast<const PairHalf<SpecFp16>::T*>(T), np, per, ts);
       break;
     default:
-      pair_spectra_kernel<PairHalf<SpecBf16>>
-          <<<grid, 256, smem, s>>>(X, nt, L, sums, static_cast<PairHalf<SpecBf16>::T*>(out), base, ts);
+      pair_sum_kernel<PairHalf<SpecBf16>>
+          <<<grid, 256, 0, s>>>(static_cast<const PairHalf<SpecBf16>::T*>(T), np, per, ts);
       break;
   }
   GISSPA_LAUNCH_CHECK();

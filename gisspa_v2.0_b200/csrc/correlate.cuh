@@ -148,7 +148,8 @@ void engine_launch(int spec, int epi, const float2* I, const void* T, const Engi
 
 // ---- sweep 1 with two templates per transform (corr_pair.cu): EPI_SUM, EPI_SUMMAX and EPI_TOPK
 // at window sizes 256, 320 and 512.  Adds the sums of squares and the maxima to the state; the
-// plain sums come from pair_sum_finish.
+// plain sums come from pair_sum_finish.  Several angles can go through one launch: "template"
+// v = a nt + t is template t at the a-th of them (args.angle or angle_state: the first).
 bool pair_supported(int L, int epi);
 // Windows and (an even number of) templates per launch.
 void pair_batch(int L, int W, int nt, int& D, int& E);
@@ -156,10 +157,10 @@ void pair_batch(int L, int W, int nt, int& D, int& E);
 // by the caller before a sweep).
 size_t pair_spectrum_bytes(int L, int spec);
 size_t pair_sum_bytes(int L);
-// Pairs' spectra of one angle from the rotated templates' half spectra X[n][kx][ky] and their
-// sums (as finalize_spectra), added to the running sum as well.
-void pair_spectra(const float2* X, int nt, int L, const double* sums, int spec, void* out, double base, void* tsum,
-                  cudaStream_t s);
+// FP16 / BF16 pairs of n images from their unscaled half spectra X[n][kx][ky] and sums.
+void pair_pack(const float2* X, int n, int L, const double* sums, int spec, void* out, double base, cudaStream_t s);
+// Adds a step's pairs (as stored) to the running sum.
+void pair_sum(const void* T, int nt, int L, int spec, void* tsum, cudaStream_t s);
 // The half spectrum (FP32) of the sum of every template-rotation since tsum was zeroed.
 void pair_sum_finish(const void* tsum, int L, float2* out, cudaStream_t s);
 // Column and row pass of cl.D templates from a.n0 (even) and cl.E windows from a.b0.

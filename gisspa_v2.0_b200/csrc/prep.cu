@@ -350,37 +350,50 @@ __device__ __forceinline__ float rotated_sample(const float* __restrict__ src, i
   return src[k0] * tt * uu + src[k1] * t * uu + src[k2] * t * u + src[k3] * tt * u;
 }
 
-__global__ void rotate_kernel(const float* __restrict__ in, int l, float cose, float sine, int mask, float d_m,
-                              float ehw, float2* __restrict__ out, double* __restrict__ sums,
-                              const AngleState* __restrict__ st) {
+// Image i of the launch: template list[i] (or i % nt) rotated by the angle of st (entry i / nt, or
+// the first with a list) or by (cose, sine), masked; its sum and sum of squares in sums[2 i].
+// A CTA takes kRotPix pixels, so that the FP64 reduction of the sums is small beside them.
+constexpr int kRotPix = 2048;
+__global__ void __launch_bounds__(kT) rotate_kernel(const float* __restrict__ in, int l, int nt,
+                                                    const int* __restrict__ list, float cose, float sine,
+                                                    const float* __restrict__ mask, float2* __restrict__ out,
+                                                    double* __restrict__ sums, const AngleState* __restrict__ st) {
   __shared__ double sh[32];
-  if (st) {
-    cose = st->cose;
-    sine = st->sine;
-  }
   const int n = blockIdx.y;
-  const int id = blockIdx.x * blockDim.x + threadIdx.x;
-  const float* src = in + (size_t)n * l * l;
-  float res = 0.f;
-  if (id < l * l) {
-    res = rotated_sample(src, l, id, cose, sine);
-    if (mask) {
-      const int i = id % l, j = id / l;
-      const float dm = 1.5f * d_m;
-      const float r = hypotf((float)(i - l / 2), (float)(j - l / 2));
-      if (r > dm / 2 + 2 * ehw) res = 0.f;
-      else if (r >= dm / 2) res *= (float)(0.5 * cos(kRefPi * (r - dm / 2) / (2.0 * ehw)) + 0.5);
-    }
+  if (st) {
+    const AngleState a = st[list ? 0 : n / nt];
+    cose = a.cose;
+    sine = a.sine;
+  }
+  const float* src = in + (size_t)(list ? list[n] : n % nt) * l * l;
+  double s1 = 0, s2 = 0;
+  const int end = min(l * l, (int)(blockIdx.x + 1) * kRotPix);
+  for (int id = blockIdx.x * kRotPix + threadIdx.x; id < end; id += kT) {
+    const float m = mask[id];
+    const float res = m == 0.f ? 0.f : rotated_sample(src, l, id, cose, sine) * m;
     out[(size_t)n * l * l + id] = make_float2(res, 0.f);
+    s1 += (double)res;
+    s2 += (double)res * res;
   }
-  if (sums) {
-    const double s1 = block_sum((double)res, sh);
-    const double s2 = block_sum((double)res * res, sh);
-    if (threadIdx.x == 0) {
-      atomicAdd(sums + 2 * n, s1);
-      atomicAdd(sums + 2 * n + 1, s2);
-    }
+  s1 = block_sum(s1, sh);
+  s2 = block_sum(s2, sh);
+  if (threadIdx.x == 0) {
+    atomicAdd(sums + 2 * n, s1);
+    atomicAdd(sums + 2 * n + 1, s2);
   }
+}
+
+// Soft circular mask of the rotated templates (apply_mask, kernels.cu:225-241) as a table.
+__global__ void mask_table_kernel(float* __restrict__ mask, int l, float d_m, float ehw) {
+  const int id = blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= l * l) return;
+  const int i = id % l, j = id / l;
+  const float dm = 1.5f * d_m;
+  const float r = hypotf((float)(i - l / 2), (float)(j - l / 2));
+  float m = 1.f;
+  if (r > dm / 2 + 2 * ehw) m = 0.f;
+  else if (r >= dm / 2) m = (float)(0.5 * cos(kRefPi * (r - dm / 2) / (2.0 * ehw)) + 0.5);
+  mask[id] = m;
 }
 
 // The norm_type=0 search rotates the windows instead of the templates: image b = a W + w of the
@@ -395,8 +408,9 @@ __global__ void rotate_windows_kernel(const float* __restrict__ in, int W, int l
 
 template <typename SPEC>
 __global__ void finalize_spectra_kernel(const float2* __restrict__ X, int l, const double* __restrict__ sums,
-                                        typename SPEC::T* __restrict__ out, double base) {
-  const int n = blockIdx.y;
+                                        typename SPEC::T* __restrict__ out, double base,
+                                        const int* __restrict__ list) {
+  const int n = blockIdx.y, to = list ? list[n] : n;
   const long long per = (long long)(l / 2 + 1) * l;
   const double L2 = (double)l * l;
   double sc = base;
@@ -410,7 +424,7 @@ __global__ void finalize_spectra_kernel(const float2* __restrict__ X, int l, con
     float2 v = X[(size_t)n * per + k];
     v = make_float2(v.x * fs, v.y * fs);
     if (sums && k == 0) v = make_float2(0.f, 0.f);  // mean subtracted: DC is exactly zero
-    out[(size_t)n * per + k] = SPEC::pack(v);
+    out[(size_t)to * per + k] = SPEC::pack(v);
   }
 }
 
@@ -524,11 +538,16 @@ void gather_windows(const float* img, int nx, int ny, const int* offx, const int
   GISSPA_LAUNCH_CHECK();
 }
 
-void rotate_batch(const float* in, int n, int l, float cose, float sine, bool mask, float d_m, float ehw, float2* out,
-                  double* sums, cudaStream_t s, const AngleState* st) {
-  if (sums) GISSPA_CUDA(cudaMemsetAsync(sums, 0, sizeof(double) * 2 * n, s));
-  rotate_kernel<<<dim3(ceil_div((long long)l * l, kT), n), kT, 0, s>>>(in, l, cose, sine, mask ? 1 : 0, d_m, ehw, out,
-                                                                       sums, st);
+void rotate_batch(const float* in, int n, int nt, const int* list, int l, float cose, float sine, const float* mask,
+                  float2* out, double* sums, cudaStream_t s, const AngleState* st) {
+  GISSPA_CUDA(cudaMemsetAsync(sums, 0, sizeof(double) * 2 * n, s));
+  rotate_kernel<<<dim3(ceil_div((long long)l * l, kRotPix), n), kT, 0, s>>>(in, l, nt, list, cose, sine, mask, out, sums,
+                                                                            st);
+  GISSPA_LAUNCH_CHECK();
+}
+
+void mask_table(float* mask, int l, float d_m, float ehw, cudaStream_t s) {
+  mask_table_kernel<<<ceil_div((long long)l * l, kT), kT, 0, s>>>(mask, l, d_m, ehw);
   GISSPA_LAUNCH_CHECK();
 }
 
@@ -538,18 +557,18 @@ void rotate_windows(const float* in, int W, int A, int l, const AngleState* tabl
 }
 
 void finalize_spectra(const float2* X, int n, int l, const double* sums, int spec, void* out, double base,
-                      cudaStream_t s) {
+                      cudaStream_t s, const int* list) {
   const long long per = (long long)(l / 2 + 1) * l;
   dim3 grid(std::min(ceil_div(per, kT), 512), n);
   switch (spec) {
     case GISSPA_SPEC_FP32:
-      finalize_spectra_kernel<SpecFp32><<<grid, kT, 0, s>>>(X, l, sums, static_cast<float2*>(out), base);
+      finalize_spectra_kernel<SpecFp32><<<grid, kT, 0, s>>>(X, l, sums, static_cast<float2*>(out), base, list);
       break;
     case GISSPA_SPEC_FP16:
-      finalize_spectra_kernel<SpecFp16><<<grid, kT, 0, s>>>(X, l, sums, static_cast<__half2*>(out), base);
+      finalize_spectra_kernel<SpecFp16><<<grid, kT, 0, s>>>(X, l, sums, static_cast<__half2*>(out), base, list);
       break;
     default:
-      finalize_spectra_kernel<SpecBf16><<<grid, kT, 0, s>>>(X, l, sums, static_cast<__nv_bfloat162*>(out), base);
+      finalize_spectra_kernel<SpecBf16><<<grid, kT, 0, s>>>(X, l, sums, static_cast<__nv_bfloat162*>(out), base, list);
       break;
   }
   GISSPA_LAUNCH_CHECK();

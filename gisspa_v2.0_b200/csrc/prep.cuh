@@ -53,11 +53,14 @@ void image_filter(float2* G, int nx, int ny, const DevParams& p, const double* r
 void gather_windows(const float* img, int nx, int ny, const int* offx, const int* offy, int bx, int nwin, int l,
                     float2* out, cudaStream_t s);
 
-// ---- rotation (rotate_subIMG kernels.cu:534-603)
-// out[n] = mask(rotate(in[n])) as complex (imag 0); sums[n] = {sum, sum of squares} (FP64)
-// st (optional): read cos/sin from device memory instead of cose/sine (graph replays).
-void rotate_batch(const float* in, int n, int l, float cose, float sine, bool mask, float d_m, float ehw, float2* out,
-                  double* sums, cudaStream_t s, const AngleState* st = nullptr);
+// ---- per-angle rotation
+// Images i < n: template list[i] (list null: i % nt) rotated, masked (a mask_table), as complex;
+// sums[2 i], sums[2 i + 1]: its sum and sum of squares.  st (optional): the angles in device memory
+// (image i at entry i / nt, the first entry with a list).
+void rotate_batch(const float* in, int n, int nt, const int* list, int l, float cose, float sine, const float* mask,
+                  float2* out, double* sums, cudaStream_t s, const AngleState* st = nullptr);
+// Soft circular mask of the rotated templates (apply_mask, kernels.cu:225-241) as a table.
+void mask_table(float* mask, int l, float d_m, float ehw, cudaStream_t s);
 // out[a W + w] = window w (real, l x l) rotated by angle a of the device table, a < A
 void rotate_windows(const float* in, int W, int A, int l, const AngleState* table, float2* out, cudaStream_t s);
 // Write spectra in the kx-major hot layout and storage precision:
@@ -65,7 +68,7 @@ void rotate_windows(const float* in, int W, int A, int l, const AngleState* tabl
 // the reference subtracts the mean first), base otherwise.  X is [n][l/2+1][l].
 // base_scale multiplies the result (1/l^2 for forward spectra of real images).
 void finalize_spectra(const float2* X, int n, int l, const double* sums, int spec, void* out, double base_scale,
-                      cudaStream_t s);
+                      cudaStream_t s, const int* list = nullptr);
 // Per-window radial RMS scale and repack: out[b][kx][ky] = F[b][ky][kx] / m_b (F is [b][l][l])
 void scale_batch(float2* F, int batch, long long per, const double* factors, cudaStream_t s);
 

@@ -13,6 +13,7 @@
 #include "prep.cuh"
 #include "project.cuh"
 #include "search.cuh"
+#include "tmpl_spectra.cuh"
 
 namespace gisspa {
 
@@ -242,25 +243,17 @@ struct ZCand {
   int q, win, arg;
 };
 
-// First node of a captured angle: the angle at the cursor becomes current, the cursor advances.
-__global__ void angle_select_kernel(const AngleState* __restrict__ table, int* __restrict__ cursor,
+// First node of a captured step: the na angles (at most 256) at the cursor become current, the
+// cursor advances.
+__global__ void angle_select_kernel(const AngleState* __restrict__ table, int* __restrict__ cursor, int na,
                                     AngleState* __restrict__ cur) {
-  *cur = table[*cursor];
-  *cursor += 1;
+  const int a = *cursor;
+  if ((int)threadIdx.x < na) cur[threadIdx.x] = table[a + threadIdx.x];
+  __syncthreads();
+  if (threadIdx.x == 0) *cursor = a + na;
 }
 
 __global__ void set_int_kernel(int* p, int v) { *p = v; }
-
-// Copies of whole per-template blocks (n4 16-byte words each) by a list of template indices:
-// dst[i] = src[list[i]] (gather) or dst[list[i]] = src[i] (scatter).
-template <bool GATHER>
-__global__ void template_copy_kernel(const uint4* __restrict__ src, const int* __restrict__ list, long long n4,
-                                     uint4* __restrict__ dst) {
-  const int i = blockIdx.y;
-  const long long from = GATHER ? list[i] : i, to = GATHER ? i : list[i];
-  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n4; k += (long long)gridDim.x * blockDim.x)
-    dst[to * n4 + k] = src[from * n4 + k];
-}
 
 // A bounded wait on an mbarrier phase that never completes (its single expected arrival is
 // never made, and no asynchronous copy targets it): the wait gives up after max_cycles and the
@@ -302,6 +295,32 @@ struct Ctx {
   DevParams p;
 };
 
+// Whether template spectra come from the two fused kernels (tmpl_spectra.cu).
+bool fused_spectra(int l, int spec) { return spec == GISSPA_SPEC_FP32 && tmpl_spectra_supported(l); }
+
+// The rotated templates' mask, laid out at the handle's first search.
+const float* rotation_mask(Ctx& c) {
+  gisspa_handle* h = c.h;
+  if (!h->mask.size()) mask_table(buf<float>(h->mask, c.L2), c.l, h->cfg.diameter, h->cfg.edge_half_width, c.s);
+  return h->mask.as<float>();
+}
+
+// The fused template spectra's inputs and scratch buffers, all templates at na angles.
+TmplSpectra spectra_args(Ctx& c, int na) {
+  gisspa_handle* h = c.h;
+  const int np = (h->nt * na + 1) / 2;
+  TmplSpectra p{};
+  p.src = h->prep_real.as<float>();
+  p.nt = h->nt;
+  p.na = na;
+  p.pre = buf<float>(h->prescale, h->nt);
+  p.mask = rotation_mask(c);
+  p.twL = h->fft.twiddles(c.l);
+  p.F = buf<float2>(h->rot, (size_t)np * c.L2);
+  p.sums = buf<double>(h->rsums, 4 * (size_t)np);
+  return p;
+}
+
 // ---- template preparation (PreprocessTemplate norm.cu:194-354 / nonorm.cu:178-344)
 void prepare_templates(Ctx& c) {
   gisspa_handle* h = c.h;
@@ -332,6 +351,8 @@ void prepare_templates(Ctx& c) {
   if (!nonorm) {
     h->fft.fft2(tb, tmp, nt, l, l, +1, 1.f, c.s);  // norm.cu:350-351, unnormalised
     real_part(tb, buf<float>(h->prep_real, (size_t)nt * c.L2), (long long)nt * c.L2, 1.f, c.s);
+    if (tmpl_spectra_supported(l) && !h->keep_whitened)  // (the adjoint makes no spectra)
+      tmpl_prescale(l, spectra_args(c, 1), buf<float>(h->prescale, nt), c.s);
   } else {
     h->fft.transpose(tb, tmp, nt, l, l, c.s, l / 2 + 1);
     void* ts = h->tspec.ensure(spec_bytes(h->cfg.spectrum_precision) * (size_t)nt * (l / 2 + 1) * l);
@@ -370,64 +391,64 @@ void window_spectra(Ctx& c, const float* img, int nx, int ny, const std::vector<
   h->fft.transpose(w, buf<float2>(h->ispec, (size_t)W * (l / 2 + 1) * l), W, l, l, c.s, l / 2 + 1);
 }
 
-// RotateTemplate (norm.cu:479-521): rotate, mask, (x - mean)/sqrt(var), FFT / l^2.
-// st (optional): take the angle from device memory (graph replays); theta is then unused.
-// Rotation by theta and forward transform of n prepared templates (src): half spectra in rot_tmp,
-// the rotated templates' sums in rsums.
-void rotated_spectra(Ctx& c, float theta, const float* src, int n, const AngleState* st) {
+// RotateTemplate (norm.cu:479-521): rotate, mask, (x - mean)/sqrt(var), FFT / l^2, for all
+// templates or those of a device list (template pairs where fused_spectra), as one half
+// spectrum per template in the storage type `spec` or as the paired correlation's pairs.
+// st (optional): take the angle from device memory (graph replays; with paired, na angles); theta is
+// then unused.
+void template_spectra(Ctx& c, float theta, const AngleState* st, int na, const int* list, int n_list, bool paired,
+                      int spec, void* out) {
   gisspa_handle* h = c.h;
-  const int l = c.l, nt = h->nt, hs = l / 2 + 1;
+  const int l = c.l, n = h->nt, hs = l / 2 + 1;
   const double rad = (double)theta * kRefPi / 180.0;
-  float2* rot = buf<float2>(h->rot, (size_t)nt * c.L2);
-  float2* rtmp = buf<float2>(h->rot_tmp, (size_t)nt * hs * l);
-  double* sums = buf<double>(h->rsums, 2 * (size_t)nt);
-  rotate_batch(src, n, l, (float)std::cos(rad), (float)std::sin(rad), true, h->cfg.diameter, h->cfg.edge_half_width,
-               rot, sums, c.s, st);
-  h->fft.rows(rot, (long long)n * l, l, -1, 1.f, c.s);
-  h->fft.transpose(rot, rtmp, n, l, l, c.s, hs);
-  h->fft.rows(rtmp, (long long)n * hs, l, -1, 1.f, c.s);
-}
-
-// The same, scaled into spectra (dst, in the storage type of the search's precision).
-void spectra_of(Ctx& c, float theta, const float* src, int n, void* dst, const AngleState* st) {
-  gisspa_handle* h = c.h;
-  rotated_spectra(c, theta, src, n, st);
-  finalize_spectra(h->rot_tmp.as<float2>(), n, c.l, h->rsums.as<double>(), h->cfg.spectrum_precision, dst,
-                   1.0 / (double)c.L2, c.s);
+  const float cose = (float)std::cos(rad), sine = (float)std::sin(rad);
+  if (fused_spectra(l, spec)) {
+    TmplSpectra p = spectra_args(c, na);
+    p.list = list;
+    p.n_list = n_list;
+    p.cose = cose;
+    p.sine = sine;
+    p.st = st;
+    p.paired = paired;
+    p.out = out;
+    tmpl_spectra(l, p, c.s);
+    return;
+  }
+  const int m = list ? n_list : n * na;  // images
+  float2* rot = buf<float2>(h->rot, (size_t)n * na * c.L2);
+  float2* rtmp = buf<float2>(h->rot_tmp, (size_t)n * na * hs * l);
+  double* sums = buf<double>(h->rsums, 2 * (size_t)n * na);
+  rotate_batch(h->prep_real.as<float>(), m, n, list, l, cose, sine, rotation_mask(c), rot, sums, c.s, st);
+  h->fft.rows(rot, (long long)m * l, l, -1, 1.f, c.s);
+  h->fft.transpose(rot, rtmp, m, l, l, c.s, hs);
+  h->fft.rows(rtmp, (long long)m * hs, l, -1, 1.f, c.s);
+  if (paired)
+    pair_pack(rtmp, m, l, sums, spec, out, 1.0 / (double)c.L2, c.s);
+  else
+    finalize_spectra(rtmp, m, l, sums, spec, out, 1.0 / (double)c.L2, c.s, list);
 }
 
 void template_spectra_at(Ctx& c, float theta, const AngleState* st = nullptr) {
   gisspa_handle* h = c.h;
-  const int l = c.l, nt = h->nt, hs = l / 2 + 1;
-  void* ts = h->tspec.ensure(spec_bytes(h->cfg.spectrum_precision) * (size_t)nt * hs * l);
-  spectra_of(c, theta, h->prep_real.as<float>(), nt, ts, st);
+  const int nt = h->nt, spec = h->cfg.spectrum_precision;
+  void* ts = h->tspec.ensure(spec_bytes(spec) * (size_t)nt * (c.l / 2 + 1) * c.l);
+  template_spectra(c, theta, st, 1, nullptr, 0, false, spec, ts);
 }
 
-// The spectra of the listed templates only, in their places among the template spectra (the
-// others keep what an earlier angle left there: the pruned second sweep reads none of them).
-// Each template's transform is independent of the others': the same values as for all.
+// The spectra of the listed templates (and their transform partners) only, in their places among
+// the template spectra (the others keep what an earlier angle left there: the pruned second sweep
+// reads none of them).  The values are those of template_spectra_at.
 void template_spectra_listed(Ctx& c, float theta, const std::vector<int>& list) {
   gisspa_handle* h = c.h;
-  const int l = c.l, nt = h->nt, hs = l / 2 + 1, n = (int)list.size();
-  if (2 * n > nt) {  // most templates: transforming all of them costs less than the copies
-    template_spectra_at(c, theta);
-    return;
-  }
-  const size_t tb = spec_bytes(h->cfg.spectrum_precision) * (size_t)hs * l;
-  float* sub = buf<float>(h->prep_sub, (size_t)nt * c.L2 / 2);  // sized for half of them: allocated once
-  char* ts_sub = static_cast<char*>(h->tspec_sub.ensure(tb * (nt / 2)));
-  char* ts = static_cast<char*>(h->tspec.ensure(tb * nt));
+  const int nt = h->nt, spec = h->cfg.spectrum_precision;
+  void* ts = h->tspec.ensure(spec_bytes(spec) * (size_t)nt * (c.l / 2 + 1) * c.l);
+  std::vector<int> want;  // (list is ascending)
+  const int per = fused_spectra(c.l, spec) ? 2 : 1;
+  for (int t : list)
+    if (want.empty() || want.back() != t / per) want.push_back(t / per);
   int* dlist = buf<int>(h->list_dev, (size_t)nt);
-  GISSPA_CUDA(cudaMemcpyAsync(dlist, list.data(), sizeof(int) * n, cudaMemcpyHostToDevice, c.s));
-  static_assert(sizeof(float) * 4 == sizeof(uint4), "16-byte words");
-  const long long w_in = (long long)c.L2 / 4, w_out = (long long)(tb / sizeof(uint4));
-  template_copy_kernel<true><<<dim3(64, n), 256, 0, c.s>>>(reinterpret_cast<const uint4*>(h->prep_real.as<float>()),
-                                                          dlist, w_in, reinterpret_cast<uint4*>(sub));
-  GISSPA_LAUNCH_CHECK();
-  spectra_of(c, theta, sub, n, ts_sub, nullptr);
-  template_copy_kernel<false><<<dim3(64, n), 256, 0, c.s>>>(reinterpret_cast<const uint4*>(ts_sub), dlist, w_out,
-                                                           reinterpret_cast<uint4*>(ts));
-  GISSPA_LAUNCH_CHECK();
+  GISSPA_CUDA(cudaMemcpyAsync(dlist, want.data(), sizeof(int) * want.size(), cudaMemcpyHostToDevice, c.s));
+  template_spectra(c, theta, nullptr, 1, dlist, (int)want.size(), false, spec, ts);
 }
 
 void choose_batches(const gisspa_config& cfg, int l, int W, int nt, int& D, int& E) {
@@ -604,15 +625,25 @@ bool sweep_paired(const gisspa_config& cfg, int l, int epi) {
          !(cfg.tensor_cores && cfg.spectrum_precision == GISSPA_SPEC_FP16 && l == 512);
 }
 
-// One angle of a paired sweep 1: template pairs' spectra (added to the running sum), then every
-// (window, template) pair.
-long long pair_angle(Ctx& c, float theta, const AngleState* st, int epi, int W, CorrArgs args) {
+// Angles per step of a paired sweep over n angles: up to 256 rotated templates together, so that a
+// few templates or windows still fill the GPU and a launch's fixed costs (each of the step's kernels
+// takes 4 to 15 us however small) are shared; at least three steps, the last ones replays of a graph.
+// A divisor of n where one is near.
+int angles_per_step(int nt, int n) {
+  const int most = std::max(1, std::min(kMaxListedTemplates / nt, n / 3));
+  for (int na = most; 2 * na > most; --na)
+    if (n % na == 0) return na;
+  return most;
+}
+
+// na angles (st, in device memory) of a paired sweep 1: template pairs' spectra (added to the
+// running sum), then every (window, template, angle).
+long long pair_angles(Ctx& c, const AngleState* st, int na, int epi, int W, CorrArgs args) {
   gisspa_handle* h = c.h;
-  const int l = c.l, nt = h->nt, spec = h->cfg.spectrum_precision;
-  rotated_spectra(c, theta, h->prep_real.as<float>(), nt, st);
+  const int l = c.l, nt = h->nt * na, spec = h->cfg.spectrum_precision;
   void* T = h->tpair.ensure(pair_spectrum_bytes(l, spec) * ((nt + 1) / 2));
-  pair_spectra(h->rot_tmp.as<float2>(), nt, l, h->rsums.as<double>(), spec, T, 1.0 / (double)c.L2,
-               h->tsum.as<void>(), c.s);
+  template_spectra(c, 0.f, st, na, nullptr, 0, true, spec, T);
+  pair_sum(T, nt, l, spec, h->tsum.as<void>(), c.s);
   int D = 1, E = 1;
   pair_batch(l, W, nt, D, E);
   float2* Q = buf<float2>(h->Q, (size_t)D * E * (l / 2) * l);
@@ -868,11 +899,11 @@ void key_put(std::vector<unsigned char>& k, const T& v) {
 
 // Everything one captured angle depends on besides the angle: shapes, buffer addresses, and the
 // epilogue's arguments (device contents such as window offsets are read at replay time).
-std::vector<unsigned char> angle_graph_key(Ctx& c, const NormRun& r, int epi) {
+std::vector<unsigned char> angle_graph_key(Ctx& c, const NormRun& r, int epi, int na) {
   gisspa_handle* h = c.h;
   const CorrArgs& a = r.args;
   std::vector<unsigned char> k;
-  for (int v : {epi, c.l, r.W, h->nt, r.D, r.E, h->cfg.spectrum_precision, a.nt_real, a.nt_total, a.bx, a.nx, a.ny})
+  for (int v : {epi, c.l, r.W, h->nt, na, r.D, r.E, h->cfg.spectrum_precision, a.nt_real, a.nt_total, a.bx, a.nx, a.ny})
     key_put(k, v);
   for (float v : {a.thresh, a.dmin, h->cfg.diameter, h->cfg.edge_half_width}) key_put(k, v);
   key_put(k, a.cand_cap);
@@ -881,6 +912,7 @@ std::vector<unsigned char> angle_graph_key(Ctx& c, const NormRun& r, int epi) {
                         (const void*)h->tspec.as<void>(), (const void*)h->ispec.as<void>(),
                         (const void*)h->Q.as<void>(), (const void*)h->gen_z.as<void>(),
                         (const void*)h->gen_x.as<void>(), (const void*)a.S1, (const void*)a.S2, (const void*)a.peak,
+                        (const void*)h->mask.as<void>(), (const void*)h->prescale.as<void>(),
                         (const void*)a.peak32, (const void*)h->tpair.as<void>(), (const void*)h->tsum.as<void>(),
                         (const void*)a.musig, (const void*)a.skip.rows, (const void*)a.skip.windows,
                         (const void*)a.skip.pairs, (const void*)a.pair_max,
@@ -892,19 +924,20 @@ std::vector<unsigned char> angle_graph_key(Ctx& c, const NormRun& r, int epi) {
   return k;
 }
 
-// Template spectra of one angle and its correlation sweep (r.args holds the angle).
-long long one_angle(Ctx& c, NormRun& r, int epi, float theta, const AngleState* st) {
+// Template spectra of one angle (of na angles from st on, in a paired sweep) and its correlation
+// sweep (r.args holds the first angle).
+long long one_step(Ctx& c, NormRun& r, int epi, float theta, const AngleState* st, int na) {
   gisspa_handle* h = c.h;
-  if (sweep_paired(h->cfg, c.l, epi)) return pair_angle(c, theta, st, epi, r.W, r.args);
+  if (sweep_paired(h->cfg, c.l, epi)) return pair_angles(c, st, na, epi, r.W, r.args);
   template_spectra_at(c, theta, st);
   return correlate_all(c, epi, h->ispec.as<float2>(), r.W, h->tspec.as<void>(), h->nt, r.args, r.D, r.E);
 }
 
 // The captured graph of one angle of this sweep (captured on first use, and again whenever its
 // key changes or any device buffer has been reallocated since).
-AngleGraph& angle_graph(Ctx& c, NormRun& r, int epi) {
+AngleGraph& angle_graph(Ctx& c, NormRun& r, int epi, int na) {
   gisspa_handle* h = c.h;
-  std::vector<unsigned char> key = angle_graph_key(c, r, epi);
+  std::vector<unsigned char> key = angle_graph_key(c, r, epi, na);
   const unsigned long long gen = alloc_generation().load();
   for (auto it = h->graphs.begin(); it != h->graphs.end();) {
     if (it->generation != gen) {  // stale addresses: never replay again
@@ -928,9 +961,9 @@ AngleGraph& angle_graph(Ctx& c, NormRun& r, int epi) {
   h->capturing = true;
   GISSPA_CUDA(cudaStreamBeginCapture(c.s, cudaStreamCaptureModeThreadLocal));
   try {
-    angle_select_kernel<<<1, 1, 0, c.s>>>(h->angle_table.as<AngleState>(), h->angle_cursor.as<int>(), cur);
+    angle_select_kernel<<<1, 256, 0, c.s>>>(h->angle_table.as<AngleState>(), h->angle_cursor.as<int>(), na, cur);
     GISSPA_LAUNCH_CHECK();
-    pairs = one_angle(c, r, epi, 0.f, cur);
+    pairs = one_step(c, r, epi, 0.f, cur, na);
   } catch (...) {
     h->capturing = false;
     r.args.angle_state = nullptr;
@@ -957,37 +990,44 @@ AngleGraph& angle_graph(Ctx& c, NormRun& r, int epi) {
   return h->graphs.back();
 }
 
-// Angles [a0, a1) of one sweep.  With cuda_graphs, the first angle runs from the host (it
-// allocates, autotunes and samples the pass timings) and the rest replay one captured graph.
+// Angles [a0, a1) of one sweep, in steps of one angle (several in a paired sweep).  With
+// cuda_graphs, the first step runs from the host (it allocates, autotunes and samples the pass
+// timings) and the other whole steps replay one captured graph.
 void run_angles(Ctx& c, NormRun& r, int epi, int a0, int a1) {
   gisspa_handle* h = c.h;
-  const bool graphs = h->cfg.cuda_graphs != 0 && a1 - a0 >= 3;
-  for (int a = a0; a < (graphs ? a0 + 1 : a1); ++a) {
-    r.args.angle = a;
-    r.args.angle_state = nullptr;
-    r.pairs += one_angle(c, r, epi, r.angles[a], nullptr);
-  }
-  if (!graphs) return;
+  if (a1 <= a0) return;
+  const bool paired = sweep_paired(h->cfg, c.l, epi);
+  const int na = paired ? angles_per_step(h->nt, a1 - a0) : 1, steps = (a1 - a0) / na;
+  const bool graphs = h->cfg.cuda_graphs != 0 && steps >= 3;
   AngleState* table = buf<AngleState>(h->angle_table, r.angles.size());
-  int* cursor = buf<int>(h->angle_cursor, 1);
-  buf<AngleState>(h->angle_cur, 1);
-  if (!r.angle_table_ready) {
+  if ((graphs || paired) && !r.angle_table_ready) {
     std::vector<AngleState>& t = r.angle_table;
     t.resize(r.angles.size());
     for (size_t a = 0; a < t.size(); ++a) {
-      const double rad = (double)r.angles[a] * kRefPi / 180.0;  // as template_spectra_at
+      const double rad = (double)r.angles[a] * kRefPi / 180.0;  // as template_spectra
       t[a] = AngleState{(int)a, (float)std::cos(rad), (float)std::sin(rad), 0};
     }
     GISSPA_CUDA(cudaMemcpyAsync(table, t.data(), sizeof(AngleState) * t.size(), cudaMemcpyHostToDevice, c.s));
     r.angle_table_ready = true;
   }
-  set_int_kernel<<<1, 1, 0, c.s>>>(cursor, a0 + 1);
-  GISSPA_LAUNCH_CHECK();
-  AngleGraph& g = angle_graph(c, r, epi);
-  for (int a = a0 + 1; a < a1; ++a) GISSPA_CUDA(cudaGraphLaunch(g.exec, c.s));
-  launch_counter() += g.launches * (a1 - a0 - 1);
-  r.pairs += g.pairs * (a1 - a0 - 1);
-  h->st.graph_replays += a1 - a0 - 1;
+  auto from_host = [&](int a, int n) {
+    r.args.angle = a;
+    r.args.angle_state = nullptr;
+    r.pairs += one_step(c, r, epi, r.angles[a], paired ? table + a : nullptr, n);
+  };
+  for (int i = 0; i < (graphs ? 1 : steps); ++i) from_host(a0 + i * na, na);
+  if (graphs) {
+    int* cursor = buf<int>(h->angle_cursor, 1);
+    buf<AngleState>(h->angle_cur, kMaxListedTemplates);
+    set_int_kernel<<<1, 1, 0, c.s>>>(cursor, a0 + na);
+    GISSPA_LAUNCH_CHECK();
+    AngleGraph& g = angle_graph(c, r, epi, na);
+    for (int i = 1; i < steps; ++i) GISSPA_CUDA(cudaGraphLaunch(g.exec, c.s));
+    launch_counter() += g.launches * (steps - 1);
+    r.pairs += g.pairs * (steps - 1);
+    h->st.graph_replays += (long long)na * (steps - 1);
+  }
+  if (a0 + steps * na < a1) from_host(a0 + steps * na, a1 - a0 - steps * na);
 }
 
 // Sweep 1 (ComputeCCGSum norm.cu:523-544) or the single top-K sweep over angles [a0, a1).
@@ -1501,10 +1541,8 @@ void debug_stage(gisspa_handle* h, int what, const float* d_img, int nx, int ny,
     return;
   }
   if (what == GISSPA_STAGE_TEMPLATE_SPECTRA) {
-    template_spectra_at(c, theta);
     float2* tmp = buf<float2>(h->tb_tmp, (size_t)h->nt * hs * l);
-    finalize_spectra(h->rot_tmp.as<float2>(), h->nt, l, h->rsums.as<double>(), GISSPA_SPEC_FP32, tmp,
-                     1.0 / (double)c.L2, c.s);
+    template_spectra(c, theta, nullptr, 1, nullptr, 0, false, GISSPA_SPEC_FP32, tmp);
     fetch(tmp, sizeof(float2) * (size_t)h->nt * hs * l);
     return;
   }

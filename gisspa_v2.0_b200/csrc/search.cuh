@@ -72,7 +72,7 @@ struct gisspa_handle {
   // template preparation
   gisspa::DevBuf tb, tb_tmp, prep_real, table, tspec;
   // per-angle rotation
-  gisspa::DevBuf rot, rot_tmp, rsums;
+  gisspa::DevBuf rot, rot_tmp, rsums, mask, prescale;
   // micrograph and windows
   gisspa::DevBuf img_in, img_c, img_tmp, img_pre, tile_real;
   gisspa::DevBuf win_c, win_tmp, win_real, ispec;
@@ -84,7 +84,7 @@ struct gisspa_handle {
   // correlation intermediate and outputs
   gisspa::DevBuf Q, cand, cand_count, nn_key, nn_sum, zkey, zcand, zcount;
   gisspa::DevBuf alive, alive_count, pair_max;  // rows and pairs sweep 2 transforms (prune_sweep2)
-  gisspa::DevBuf prep_sub, tspec_sub, list_dev;  // the live templates of an angle of that sweep
+  gisspa::DevBuf list_dev;  // the live templates of an angle of that sweep
   gisspa::DevBuf engine_ctr;  // work counters of the pair engine, one block per launch of a sequence
   // paired sweep 1: template pairs' spectra of an angle, the running sum of all templates' spectra,
   // that sum as one FP32 half spectrum, and its correlation maps
