@@ -10,15 +10,18 @@
 // prefixes keep k inside the binade (by one unit at either end) has the result k + D0 (+ d); the
 // additions that leave it are done one by one.
 //
-//   1. chunk_sum_kernel: FP64 sums of 1024-term chunks (only to choose binades)
+//   1. block_sum_kernel: FP64 sums of 4096-term blocks (only to choose binades)
 //   2. binade_kernel: the largest running sum's exponent
-//   3. chunk_map_kernel: every chunk's map in the kBinades binades below it
-//   4. walk_kernel: one CTA per sum composes 256 chunks at a time and takes those that fit; the
-//      first that does not is added term by term
+//   3. chunk_map_kernel, block_map_kernel: the maps of every 256-term chunk and every block in the
+//      kBinades binades below it
+//   4. walk_kernel: one CTA per sum composes 256 blocks at a time and takes those that fit; the
+//      first that does not goes chunk by chunk, and the chunks that leave the binade term by term
 // One thread adding the 16.8 M terms of a 4096^2 micrograph took 65 ms (a dependent FP32 addition
-// per term).  This takes 0.7 ms where the mean is well away from zero and 13 ms for a zero-mean
+// per term).  This takes 0.6 ms where the mean is well away from zero and 10.6 ms for a zero-mean
 // micrograph, whose running sum changes its binade often: the chunks in which it does (a serial
-// chain of 1024 additions each) bound it.  2048^2: 0.24 and 3.8 ms instead of 16.
+// chain of 256 additions each) bound it.  2048^2: 0.23 and 3.0 ms instead of 16.
+// (Blocks of one size only, 1024 terms: 13.5 and 3.8 ms.  Maps of 16 terms for the failing part: 36 ms,
+// one warp's checks cost more than the additions that they save.)
 #include <cmath>
 
 #include "prep.cuh"
@@ -26,10 +29,12 @@
 namespace gisspa {
 namespace {
 
-constexpr int kChunk = 1024, kLane = kChunk / 32;  // terms per chunk, per lane
+constexpr int kChunk = 256, kPerLane = 32;         // terms per chunk, per lane of step 3
+constexpr int kLanes = kChunk / kPerLane;           // lanes per chunk
+constexpr int kBlock = 4096, kCB = kBlock / kChunk;  // terms per block, chunks per block
 constexpr int kBinades = 16;
 constexpr int kOut = 1 << 29;  // a bound no prefix may reach
-constexpr int kWarps = 8;      // chunks per CTA of step 3
+constexpr int kWarps = 8;      // warps per CTA of step 3
 
 // The terms of the two sums (norm.cu:160-163) with the reference's roundings.
 __device__ __forceinline__ float term1(float v, float fnx, float fny) { return __fdiv_rn(__fdiv_rn(v, fnx), fny); }
@@ -80,24 +85,25 @@ __device__ __forceinline__ RunMap shfl_up_map(const RunMap& m, int o) {
   return RunMap{__shfl_up_sync(0xffffffffu, m.D0, o), __shfl_up_sync(0xffffffffu, m.d, o),
                 __shfl_up_sync(0xffffffffu, m.mn, o), __shfl_up_sync(0xffffffffu, m.mx, o)};
 }
-// Inclusive composition over the lanes, in lane order.
+// Inclusive composition over each group of W lanes, in lane order.
+template <int W = 32>
 __device__ __forceinline__ RunMap scan_map(RunMap m, int lane) {
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
+  for (int o = 1; o < W; o <<= 1) {
     const RunMap p = shfl_up_map(m, o);
-    if (lane >= o) m = compose(p, m);
+    if ((lane & (W - 1)) >= o) m = compose(p, m);
   }
   return m;
 }
 
-__global__ void __launch_bounds__(256) chunk_sum_kernel(const float* __restrict__ img, long long n, float fnx,
-                                                        float fny, double* __restrict__ sums, int nchunks) {
+__global__ void __launch_bounds__(256) block_sum_kernel(const float* __restrict__ img, long long n, float fnx,
+                                                        float fny, double* __restrict__ sums, int nblocks) {
   const int c = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (c >= nchunks) return;
+  if (c >= nblocks) return;
   double a = 0, b = 0;
-  const long long base = (long long)c * kChunk;
+  const long long base = (long long)c * kBlock;
 #pragma unroll 8
-  for (int i = lane; i < kChunk; i += 32)
+  for (int i = lane; i < kBlock; i += 32)
     if (base + i < n) {
       const float v = img[base + i];
       a += v;
@@ -110,20 +116,20 @@ __global__ void __launch_bounds__(256) chunk_sum_kernel(const float* __restrict_
   if (lane == 0) {
     const double s = 1.0 / ((double)fnx * fny);
     sums[c] = a * s;
-    sums[nchunks + c] = b * s;
+    sums[nblocks + c] = b * s;
   }
 }
 
 // etop[j]: the exponent of the largest running sum j, plus one for the drift of the rounded sum.
-__global__ void __launch_bounds__(1024) binade_kernel(const double* __restrict__ sums, int nchunks,
+__global__ void __launch_bounds__(1024) binade_kernel(const double* __restrict__ sums, int nblocks,
                                                       int* __restrict__ etop) {
   __shared__ double sh[1024];
   __shared__ double big[32];
   for (int j = 0; j < 2; ++j) {
     // each thread a contiguous run: its total, then the prefixes inside it
-    const int per = (nchunks + 1023) / 1024, c0 = threadIdx.x * per, c1 = min(nchunks, c0 + per);
+    const int per = (nblocks + 1023) / 1024, c0 = threadIdx.x * per, c1 = min(nblocks, c0 + per);
     double t = 0;
-    for (int c = c0; c < c1; ++c) t += sums[(size_t)j * nchunks + c];
+    for (int c = c0; c < c1; ++c) t += sums[(size_t)j * nblocks + c];
     sh[threadIdx.x] = t;
     __syncthreads();
     for (int o = 1; o < 1024; o <<= 1) {
@@ -134,7 +140,7 @@ __global__ void __launch_bounds__(1024) binade_kernel(const double* __restrict__
     }
     double p = sh[threadIdx.x] - t, m = 0;
     for (int c = c0; c < c1; ++c) {
-      p += sums[(size_t)j * nchunks + c];
+      p += sums[(size_t)j * nblocks + c];
       m = fmax(m, fabs(p));
     }
     for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -154,19 +160,20 @@ __device__ __forceinline__ float unit_inv(int e) { return __uint_as_float((unsig
 __global__ void __launch_bounds__(kWarps * 32) chunk_map_kernel(const float* __restrict__ img, long long n, float fnx,
                                                                 float fny, const int* __restrict__ etop,
                                                                 int4* __restrict__ tab, int nchunks) {
-  __shared__ float t[kWarps][kChunk + 32];  // one pad per lane's run: the runs' stride is odd
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.x * kWarps + w, j = blockIdx.y;
-  if (c >= nchunks) return;
-  const long long base = (long long)c * kChunk;
+  constexpr int kTerms = 32 * kPerLane;       // a warp's
+  __shared__ float t[kWarps][kTerms + 32];  // one pad per lane's run: the runs' stride is odd
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, j = blockIdx.y;
+  const long long base = ((long long)blockIdx.x * kWarps + w) * kTerms;
+  if (base / kChunk >= nchunks) return;
 #pragma unroll 4
-  for (int i = lane; i < kChunk; i += 32) {
+  for (int i = lane; i < kTerms; i += 32) {
     float v = 0.f;
     if (base + i < n) v = j ? term2(img[base + i], fnx, fny) : term1(img[base + i], fnx, fny);
-    t[w][i + i / kLane] = v;  // past the end: zeros, which change nothing
+    t[w][i + i / kPerLane] = v;  // past the end: zeros, which change nothing
   }
   __syncwarp();
-  const int e0 = etop[j];
-  const float* mine = &t[w][lane * (kLane + 1)];
+  const int e0 = etop[j], c = (int)(base / kChunk) + lane / kLanes;
+  const float* mine = &t[w][lane * (kPerLane + 1)];
 #pragma unroll 1
   for (int b0 = 0; b0 < kBinades; b0 += 4) {
     RunMap m[4];
@@ -176,17 +183,30 @@ __global__ void __launch_bounds__(kWarps * 32) chunk_map_kernel(const float* __r
       m[b] = identity_map();
       inv[b] = unit_inv(e0 - b0 - b);
     }
-    for (int i = 0; i < kLane; ++i) {
+    for (int i = 0; i < kPerLane; ++i) {
       const float v = mine[i];
 #pragma unroll
       for (int b = 0; b < 4; ++b) append(m[b], v, inv[b]);
     }
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
-      const RunMap s = scan_map(m[b], lane);
-      if (lane == 31) tab[((size_t)j * kBinades + b0 + b) * nchunks + c] = make_int4(s.D0, s.d, s.mn, s.mx);
+      const RunMap s = scan_map<kLanes>(m[b], lane);
+      if ((lane & (kLanes - 1)) == kLanes - 1 && c < nchunks)
+        tab[((size_t)j * kBinades + b0 + b) * nchunks + c] = make_int4(s.D0, s.d, s.mn, s.mx);
     }
   }
+}
+
+__device__ __forceinline__ RunMap to_map(int4 v) { return RunMap{v.x, v.y, v.z, v.w}; }
+
+// The maps of whole blocks (nchunks: whole blocks of chunks).
+__global__ void block_map_kernel(const int4* __restrict__ chunks, int nblocks, int4* __restrict__ blocks) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= 2 * kBinades * nblocks) return;
+  RunMap m = identity_map();
+#pragma unroll
+  for (int q = 0; q < kCB; ++q) m = compose(m, to_map(chunks[(size_t)i * kCB + q]));
+  blocks[i] = make_int4(m.D0, m.d, m.mn, m.mx);
 }
 
 // k, e of a normal s (false for zero, subnormals, infinities and NaN, and outside |e| <= 100).
@@ -206,9 +226,10 @@ __device__ __forceinline__ bool fits(int k, const RunMap& m) {
   return k > 0 ? (k + m.mn >= lo && k + m.mx <= hi) : (k + m.mx <= -lo && k + m.mn >= -hi);
 }
 
-constexpr int kWalk = 256, kRun = kChunk / kWalk;  // threads of step 4, terms per thread of a chunk
+constexpr int kWalk = 256;  // threads of step 4
 struct WalkShared {
-  float t[kChunk];
+  float t[kBlock];
+  int4 map[kCB][3];  // a block's chunks, in the sum's binade and the two beside it
   RunMap tot[kWalk / 32];
   int bad[kWalk / 32];
   float s;
@@ -238,56 +259,80 @@ __device__ __forceinline__ int take(WalkShared& sh, float& s, int k, int e, cons
 }
 
 __global__ void __launch_bounds__(kWalk) walk_kernel(const float* __restrict__ img, long long n, float fnx, float fny,
-                                                     const int* __restrict__ etop, const int4* __restrict__ tab,
-                                                     int nchunks, float* __restrict__ out) {
+                                                     const int* __restrict__ etop, const int4* __restrict__ chunks,
+                                                     const int4* __restrict__ blocks, int nblocks,
+                                                     float* __restrict__ out) {
   __shared__ __align__(16) WalkShared sh;
   const int tid = threadIdx.x, j = blockIdx.x, e0 = etop[j];
-  const int4* tj = tab + (size_t)j * kBinades * nchunks;
+  const int4* tc = chunks + (size_t)j * kBinades * nblocks * kCB;
+  const int4* tb = blocks + (size_t)j * kBinades * nblocks;
   float s = 0.f;  // (the same in every thread)
   int c = 0;
-  while (c < nchunks) {
+  while (c < nblocks) {
     int k, e;
     const bool normal = split(s, k, e);
     const int b = e0 - e;
     if (normal && b >= 0 && b < kBinades) {
       RunMap m = identity_map();
-      if (c + tid < nchunks) {
-        const int4 v = tj[(size_t)b * nchunks + c + tid];
-        m = RunMap{v.x, v.y, v.z, v.w};
-      } else {
-        m.mx = kOut;  // past the last chunk
-      }
+      if (c + tid < nblocks)
+        m = to_map(tb[(size_t)b * nblocks + c + tid]);
+      else
+        m.mx = kOut;  // past the last block
       const int done = take(sh, s, k, e, m);
       c += done;
-      if (done == kWalk || c >= nchunks) continue;
+      if (done == kWalk || c >= nblocks) continue;
     }
-    // chunk c leaves the binade: its terms one by one (a sum that hovers at a power of two crosses it
-    // many times in a chunk, and finding each crossing costs more than the additions)
-    const long long base = (long long)c * kChunk;
-    float v[kRun];
+    // block c leaves the binade: its terms and its chunks' maps
+    const bool ours = split(s, k, e);
+    const long long base = (long long)c * kBlock;
+    {
+      constexpr int kEach = kBlock / kWalk;
+      float v[kEach];
 #pragma unroll
-    for (int q = 0; q < kRun; ++q) {
-      const long long at = base + tid + q * kWalk;
-      v[q] = at < n ? img[at] : 0.f;
-    }
-#pragma unroll
-    for (int q = 0; q < kRun; ++q) sh.t[tid + q * kWalk] = j ? term2(v[q], fnx, fny) : term1(v[q], fnx, fny);
-    __syncthreads();
-    if (tid < 32) {
-      const float4* t = reinterpret_cast<const float4*>(sh.t);
-      float4 x[4], y[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) x[q] = t[q];
-#pragma unroll 1
-      for (int i = 4; i <= kChunk / 4; i += 4) {  // the next 16 terms load while these are added
-#pragma unroll
-        for (int q = 0; q < 4; ++q) y[q] = t[min(i + q, kChunk / 4 - 1)];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, x[q].x), x[q].y), x[q].z), x[q].w);
-          x[q] = y[q];
-        }
+      for (int q = 0; q < kEach; ++q) {
+        const long long at = base + tid + q * kWalk;
+        v[q] = at < n ? img[at] : 0.f;
       }
+      if (tid < 3 * kCB) {
+        const int q = tid / 3, b3 = e0 - (e - 1 + tid % 3);
+        int4 m = make_int4(0, 0, 0, kOut);  // no map of this binade: not taken
+        if (ours && b3 >= 0 && b3 < kBinades) m = tc[((size_t)b3 * nblocks + c) * kCB + q];
+        sh.map[q][tid % 3] = m;
+      }
+#pragma unroll
+      for (int q = 0; q < kEach; ++q) sh.t[tid + q * kWalk] = j ? term2(v[q], fnx, fny) : term1(v[q], fnx, fny);
+    }
+    __syncthreads();
+    if (tid < 32) {  // one warp, every lane the same
+      const int eb = e;
+      bool ok = ours;  // k, e hold the sum
+#pragma unroll 1
+      for (int q = 0; q < kCB; ++q) {
+        if (ok) {
+          const RunMap m = to_map(sh.map[q][e - eb + 1]);
+          if (fits(k, m)) {
+            k += m.D0 + ((k & 1) ? m.d : 0);
+            continue;
+          }
+          s = join(k, e);
+        }
+        const float4* t = reinterpret_cast<const float4*>(sh.t + q * kChunk);
+        float4 x[4], y[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = t[i];
+#pragma unroll 4
+        for (int r = 4; r <= kChunk / 4; r += 4) {  // the next 16 terms load while these are added
+#pragma unroll
+          for (int i = 0; i < 4; ++i) y[i] = t[min(r + i, kChunk / 4 - 1)];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, x[i].x), x[i].y), x[i].z), x[i].w);
+            x[i] = y[i];
+          }
+        }
+        ok = split(s, k, e) && ours && e >= eb - 1 && e <= eb + 1;
+      }
+      if (ok) s = join(k, e);
       if (tid == 0) sh.s = s;
     }
     __syncthreads();
@@ -309,30 +354,35 @@ __global__ void stats_finish_kernel(const float* __restrict__ sums, float* __res
   if (!(up == up) || !(lo == lo)) stats[3] = 0.f;
 }
 
-int chunks_of(long long n) { return (int)((n + kChunk - 1) / kChunk); }
+int blocks_of(long long n) { return (int)((n + kBlock - 1) / kBlock); }
 
 }  // namespace
 
 size_t serial_stats_bytes(long long n) {
-  // maps, FP64 chunk sums, exponents and the two sums
-  return (size_t)chunks_of(n) * (2 * kBinades * sizeof(int4) + 2 * sizeof(double)) + 16;
+  // maps of chunks and blocks, FP64 block sums, exponents and the two sums
+  return (size_t)blocks_of(n) * (2 * kBinades * (kCB + 1) * sizeof(int4) + 2 * sizeof(double)) + 16;
 }
 
 void serial_stats(const float* img, int nx, int ny, float* stats, void* scratch, cudaStream_t s) {
   const long long n = (long long)nx * ny;
-  const int nc = chunks_of(n);
-  int4* tab = static_cast<int4*>(scratch);
-  double* sums = reinterpret_cast<double*>(tab + (size_t)2 * kBinades * nc);
-  int* etop = reinterpret_cast<int*>(sums + 2 * (size_t)nc);
+  const int nb = blocks_of(n), nc = nb * kCB;
+  int4* chunks = static_cast<int4*>(scratch);
+  int4* blocks = chunks + (size_t)2 * kBinades * nc;
+  double* sums = reinterpret_cast<double*>(blocks + (size_t)2 * kBinades * nb);
+  int* etop = reinterpret_cast<int*>(sums + 2 * (size_t)nb);
   float* out = reinterpret_cast<float*>(etop + 2);
   const float fnx = (float)nx, fny = (float)ny;
-  chunk_sum_kernel<<<ceil_div(nc, 8), 256, 0, s>>>(img, n, fnx, fny, sums, nc);
+  block_sum_kernel<<<ceil_div(nb, 8), 256, 0, s>>>(img, n, fnx, fny, sums, nb);
   GISSPA_LAUNCH_CHECK();
-  binade_kernel<<<1, 1024, 0, s>>>(sums, nc, etop);
+  binade_kernel<<<1, 1024, 0, s>>>(sums, nb, etop);
   GISSPA_LAUNCH_CHECK();
-  chunk_map_kernel<<<dim3(ceil_div(nc, kWarps), 2), kWarps * 32, 0, s>>>(img, n, fnx, fny, etop, tab, nc);
+  // (whole blocks: the last one's chunks past the image are zeros)
+  chunk_map_kernel<<<dim3(ceil_div((long long)nb * kBlock, kWarps * 32 * kPerLane), 2), kWarps * 32, 0, s>>>(
+      img, n, fnx, fny, etop, chunks, nc);
   GISSPA_LAUNCH_CHECK();
-  walk_kernel<<<2, kWalk, 0, s>>>(img, n, fnx, fny, etop, tab, nc, out);
+  block_map_kernel<<<ceil_div(2 * kBinades * nb, 128), 128, 0, s>>>(chunks, nb, blocks);
+  GISSPA_LAUNCH_CHECK();
+  walk_kernel<<<2, kWalk, 0, s>>>(img, n, fnx, fny, etop, chunks, blocks, nb, out);
   GISSPA_LAUNCH_CHECK();
   stats_finish_kernel<<<1, 1, 0, s>>>(out, stats);
   GISSPA_LAUNCH_CHECK();

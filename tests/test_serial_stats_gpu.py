@@ -1,7 +1,7 @@
 """LoadImage statistics: the reference's running FP32 sums evaluated in parallel, against the
 oracle's serial loop, on micrographs whose outlier bounds (integers, from those sums) decide which
 pixels are replaced: sums that drift by their own rounding, that hover around zero, that stay zero
-for a while or whose terms are exact ties; sizes around a chunk of 1024 terms."""
+for a while or whose terms are exact ties; sizes around a chunk of 256 and a block of 4096 terms."""
 import numpy as np
 import pytest
 
@@ -29,7 +29,7 @@ def _image(kind, shape, rng):
     return x
 
 
-@pytest.mark.parametrize("shape", [(32, 32), (31, 33), (300, 211), (1024, 1024)])
+@pytest.mark.parametrize("shape", [(32, 32), (31, 33), (64, 64), (63, 65), (300, 211), (1024, 1024)])
 @pytest.mark.parametrize("kind", ["noise", "counts", "ties", "late", "alternating"])
 def test_serial_statistics_match_the_serial_loop(kind, shape):
     rng = np.random.default_rng(len(kind) + shape[1])
