@@ -36,8 +36,9 @@ struct GradArgs {
 void ctf_dweight(float* dtab, int l, const DevParams& p, cudaStream_t s);
 // out[t] = F[t] * tab / m[t]
 void scale_by_table(const float2* F, const float* tab, const double* m, int nt, int l, float2* out, cudaStream_t s);
+// work: reduce_bytes(l, nwin)
 void window_sums(const float* img, int nx, int ny, const int* offx, const int* offy, int bx, int nwin, int l,
-                 const double* win_m, double* out, cudaStream_t s);
+                 const double* win_m, double* out, double* work, cudaStream_t s);
 // prep (n1 values) and dprep (n2) rounded to the template precision (1: FP16, 2: BF16) into out1,
 // out2; FP16 first scales both by one power of two that fits their largest value (absmax: one
 // unsigned of device scratch)

@@ -14,9 +14,13 @@ struct DevParams {
 DevParams make_params(const gisspa_config& c, const gisspa_ctf& ctf);
 
 // ---- templates
-void tmpl_pad(const float* stack, int nt, int tw, int th, int l, float2* out, cudaStream_t s);
-// edge mean over the ring + sigma over the padded window, then t <- (t - em) / sigma
-void tmpl_edge_normalise(float2* tb, int nt, int l, double* scratch, cudaStream_t s);
+// Per-image reductions: threads per CTA, CTAs per l x l image (at most kReduce; 8 pixels per thread
+// below that), and their scratch (FP64 partial sums).
+constexpr int kReduce = 256;
+int reduce_parts(int l);
+size_t reduce_bytes(int l, int batch);
+// pad to l x l; edge mean over the ring + sigma over the padded window, then t <- (t - em) / sigma
+void tmpl_normalise(const float* stack, int nt, int tw, int th, int l, float2* out, double* work, cudaStream_t s);
 // radial power over x <= nx/2, 0 <= r < max(nx, ny)/2: ra[b][r] += |F|^2, rb[r] += 1 (rb shared)
 void radial_power(const float2* F, int batch, int nx, int ny, double* ra, unsigned* rb, int nbins, cudaStream_t s);
 // F /= sqrt(ra / rb) on valid shells (whiten_Tmp kernels.cu:128-149)
@@ -27,8 +31,8 @@ void mask_real(float2* data, int batch, int l, float d_m, float ehw, cudaStream_
 void tmpl_weight_table(float* table, int l, const DevParams& p, cudaStream_t s);
 void apply_table(float2* F, int batch, int l, const float* table, cudaStream_t s);
 // F /= m, m = sqrt(sum |F|^2 / count^2) over x <= l/2 and valid shells (kernels.cu:319-382 +
-// host); m per batch entry is written to factors when not null
-void rms_normalise(float2* F, int batch, int l, double* factors, cudaStream_t s);
+// host); m per batch entry is written to factors when not null.  half: half spectra [x <= l/2][y]
+void rms_normalise(float2* F, int batch, int l, bool half, double* factors, double* work, cudaStream_t s);
 void real_part(const float2* in, float* out, long long n, float scale, cudaStream_t s);
 void to_complex(const float* in, float2* out, long long n, cudaStream_t s);
 

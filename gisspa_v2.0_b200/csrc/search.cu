@@ -328,8 +328,8 @@ void prepare_templates(Ctx& c) {
   const bool nonorm = h->cfg.norm_type == 0;
   float2* tb = buf<float2>(h->tb, (size_t)nt * c.L2);
   float2* tmp = buf<float2>(h->tb_tmp, (size_t)nt * c.L2);
-  tmpl_pad(h->d_stack.as<float>(), nt, h->tw, h->th, l, tb, c.s);
-  tmpl_edge_normalise(tb, nt, l, nullptr, c.s);
+  double* work = static_cast<double*>(h->reduce.ensure(reduce_bytes(l, nt)));
+  tmpl_normalise(h->d_stack.as<float>(), nt, h->tw, h->th, l, tb, work, c.s);
   h->fft.fft2(tb, tmp, nt, l, l, -1, 1.0f / (float)c.L2, c.s);
   const int nb = l / 2;
   double* ra = buf<double>(h->ra, (size_t)nt * nb);
@@ -347,7 +347,7 @@ void prepare_templates(Ctx& c) {
   float* table = buf<float>(h->table, c.L2);
   tmpl_weight_table(table, l, c.p, c.s);
   apply_table(tb, nt, l, table, c.s);
-  rms_normalise(tb, nt, l, buf<double>(h->tmpl_m, nt), c.s);
+  rms_normalise(tb, nt, l, false, buf<double>(h->tmpl_m, nt), work, c.s);
   if (!nonorm) {
     h->fft.fft2(tb, tmp, nt, l, l, +1, 1.f, c.s);  // norm.cu:350-351, unnormalised
     real_part(tb, buf<float>(h->prep_real, (size_t)nt * c.L2), (long long)nt * c.L2, 1.f, c.s);
@@ -383,12 +383,16 @@ void window_spectra(Ctx& c, const float* img, int nx, int ny, const std::vector<
   int* doy = buf<int>(h->offy, oy.size());
   GISSPA_CUDA(cudaMemcpyAsync(dox, ox.data(), sizeof(int) * ox.size(), cudaMemcpyHostToDevice, c.s));
   GISSPA_CUDA(cudaMemcpyAsync(doy, oy.data(), sizeof(int) * oy.size(), cudaMemcpyHostToDevice, c.s));
+  const int hs = l / 2 + 1;
   float2* w = buf<float2>(h->win_c, (size_t)W * c.L2);
-  float2* tmp = buf<float2>(h->win_tmp, (size_t)W * c.L2);
+  float2* I = buf<float2>(h->ispec, (size_t)W * hs * l);
   gather_windows(img, nx, ny, dox, doy, bx, W, l, w, c.s);
-  h->fft.fft2(w, tmp, W, l, l, -1, 1.0f / (float)c.L2, c.s);
-  rms_normalise(w, W, l, buf<double>(h->win_m, W), c.s);
-  h->fft.transpose(w, buf<float2>(h->ispec, (size_t)W * (l / 2 + 1) * l), W, l, l, c.s, l / 2 + 1);
+  // the column transforms of the half that is kept, in its layout
+  h->fft.rows(w, (long long)W * l, l, -1, 1.f, c.s);
+  h->fft.transpose(w, I, W, l, l, c.s, hs);
+  h->fft.rows(I, (long long)W * hs, l, -1, 1.0f / (float)c.L2, c.s);
+  rms_normalise(I, W, l, true, buf<double>(h->win_m, W), static_cast<double*>(h->reduce.ensure(reduce_bytes(l, W))),
+                c.s);
 }
 
 // RotateTemplate (norm.cu:479-521): rotate, mask, (x - mean)/sqrt(var), FFT / l^2, for all
@@ -1407,7 +1411,7 @@ void search_nonorm(Ctx& c, const float* d_img, int nx, int ny, std::vector<gissp
     gather_windows(tile, ts, ts, dtx, dty, bx, W, l, w, c.s);
     if (cfg.phase_flip == 1) {
       h->fft.fft2(w, wtmp, W, l, l, -1, 1.0f / (float)c.L2, c.s);
-      rms_normalise(w, W, l, nullptr, c.s);
+      rms_normalise(w, W, l, false, nullptr, static_cast<double*>(h->reduce.ensure(reduce_bytes(l, W))), c.s);
       h->fft.fft2(w, wtmp, W, l, l, +1, 1.f, c.s);
     }
     float* wr = buf<float>(h->win_real, (size_t)W * c.L2);
@@ -1597,7 +1601,8 @@ void adjoint_prepare(gisspa_handle* h, const gisspa_ctf& ctf) {
     real_part(tb, dprep + (size_t)q * nt * c.L2, (long long)nt * c.L2, 1.f, c.s);
   }
   window_sums(h->img_pre.as<float>(), h->last_nx, h->last_ny, h->offx.as<int>(), h->offy.as<int>(), h->last_bx,
-              h->last_W, l, h->win_m.as<double>(), buf<double>(h->win_sum, h->last_W), c.s);
+              h->last_W, l, h->win_m.as<double>(), buf<double>(h->win_sum, h->last_W),
+              static_cast<double*>(h->reduce.ensure(reduce_bytes(l, h->last_W))), c.s);
   // the FP16 / BF16 template forms evaluate from templates stored at that precision
   const int prec = h->cfg.spectrum_precision;
   if (prec != GISSPA_SPEC_FP32)

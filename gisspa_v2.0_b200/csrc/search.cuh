@@ -78,7 +78,7 @@ struct gisspa_handle {
   gisspa::DevBuf win_c, win_tmp, win_real, ispec;
   gisspa::DevBuf offx, offy;
   // shells, statistics
-  gisspa::DevBuf ra, rb, stats, scratch;
+  gisspa::DevBuf ra, rb, stats, scratch, reduce;
   // per-window-pixel state
   gisspa::DevBuf S1, S2, peak, peak32, musig;
   // correlation intermediate and outputs
