@@ -136,7 +136,7 @@ __global__ void window_sum_finish(const double* __restrict__ part, int parts, in
 // its derivative in the sampling coordinates.
 __device__ __forceinline__ void bilinear(int l, double x2, double y2, int& k0, int& k1,
                                          int& k2, int& k3, double& t, double& u, bool& inside) {
-  inside = !(x2 < 0 || x2 > l - 1.0 || y2 < 0 || y2 > l - 1.0);
+  inside = x2 >= 0 && x2 <= l - 1.0 && y2 >= 0 && y2 <= l - 1.0;
   if (!inside) return;
   const int ii = (int)floor(x2), jj = (int)floor(y2);
   k0 = ii + jj * l;
@@ -155,9 +155,45 @@ __device__ __forceinline__ void bilinear(int l, double x2, double y2, int& k0, i
   u = y2 - jj;
 }
 
-__device__ __forceinline__ double to_d(float v) { return (double)v; }
-__device__ __forceinline__ double to_d(__half v) { return (double)__half2float(v); }
-__device__ __forceinline__ double to_d(__nv_bfloat16 v) { return (double)__bfloat162float(v); }
+// A template pixel's table entry: the prepared template and its CTF derivatives side by side, so
+// that a bilinear corner is one load.
+template <typename V>
+struct GradPixel;
+template <>
+struct GradPixel<float> {
+  using T = float4;
+  __device__ __forceinline__ static float4 load(const T* p) { return __ldg(p); }
+};
+template <>
+struct GradPixel<__half> {
+  using T = uint2;
+  __device__ __forceinline__ static float4 load(const T* p) {
+    const uint2 r = __ldg(p);
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&r.x));
+    const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&r.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+  }
+};
+template <>
+struct GradPixel<__nv_bfloat16> {
+  using T = uint2;
+  __device__ __forceinline__ static float4 load(const T* p) {
+    const uint2 r = __ldg(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+  }
+};
+
+template <typename T>
+__global__ void plane_kernel(const T* __restrict__ in, long long n, float* __restrict__ table) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  if constexpr (std::is_same<T, float2>::value)
+    table[4 * i] = in[i].x;
+  else
+    table[4 * i] = in[i];
+}
 
 // Largest |value| of in[0, n), as the bits of a non-negative float (ordered like the value),
 // folded into *out.
@@ -171,7 +207,7 @@ __global__ void abs_max_kernel(const float* __restrict__ in, long long n, unsign
 
 // Rounds to V.  FP16 has five exponent bits: the unnormalised real-space templates and their CTF
 // derivatives exceed its range, so every value is first scaled by one power of two that brings
-// the largest (*absmax, over both arrays) to [2^13, 2^14).  A common factor leaves the
+// the largest (*absmax, over the whole table) to [2^13, 2^14).  A common factor leaves the
 // normalised score and all its derivatives unchanged (the score is invariant to the template's
 // scale), and a power of two adds no rounding.  BF16 keeps FP32's exponent range (absmax null).
 template <typename V>
@@ -190,12 +226,17 @@ __global__ void round_kernel(const float* __restrict__ in, long long n, const un
     out[i] = __float2bfloat16_rn(in[i] * scale);
 }
 
-// V: storage type of the prepared templates and their CTF derivatives (float, __half or
-// __nv_bfloat16); every sum is FP64 whatever the storage.
+// One CTA per pick, a warp per 8 x 4 tile of the mask's square: the rotated samples of a tile lie in
+// a few rows of the template whatever the angle (those of 32 pixels of a row lie in up to 32), and
+// the corners' loads are what bounds the kernel beside the FP64 arithmetic.  The mask's cosine is
+// evaluated in its ring only.  With rows of 32 pixels, a load per corner and array, and the ring's
+// expressions everywhere, 2000 picks of window 512 took 2.09 ms; now 1.16.
+// V: storage type of the table (float, __half or __nv_bfloat16); every sum is FP64 whatever the
+// storage.
 template <typename V>
-__global__ void __launch_bounds__(kGT) score_grad_kernel(GradArgs g, const V* __restrict__ prep,
-                                                         const V* __restrict__ dprep,
-                                                         const GradPick* __restrict__ picks, float* __restrict__ out) {
+__global__ void __launch_bounds__(kGT, 2) score_grad_kernel(GradArgs g, const GradPick* __restrict__ picks,
+                                                            float* __restrict__ out) {
+  using GP = GradPixel<V>;
   __shared__ double sh[kSums][kGT / 32];
   const GradPick pk = picks[blockIdx.x];
   const int L = g.L;
@@ -203,60 +244,72 @@ __global__ void __launch_bounds__(kGT) score_grad_kernel(GradArgs g, const V* __
   const double th = (double)pk.theta * kRefPi / 180.0;
   const double cs = cos(th), sn = sin(th);
   const double dm = 1.5 * g.d_m, r_in = dm / 2, r_out = dm / 2 + 2 * g.ehw;
-  const V* P = prep + (size_t)pk.n * L * L;
-  const V* D0 = dprep + (size_t)pk.n * L * L;
-  const size_t dstride = (size_t)g.nt * L * L;
+  const double in2 = r_in * r_in, out2 = r_out * r_out, karg = kRefPi / (2.0 * g.ehw);
+  const typename GP::T* P = static_cast<const typename GP::T*>(g.table) + (size_t)pk.n * L * L;
   const int wx0 = g.offx[pk.b % g.bx], wy0 = g.offy[pk.b / g.bx];
   const double wscale = 1.0 / (L2 * (g.win_m[pk.b] != 0 ? g.win_m[pk.b] : 1.0));
   const double cx = L / 2 + (double)pk.dx, cy = L / 2 + (double)pk.dy;
   const int x_lo = max(0, (int)floor(cx - r_out) - 1), x_hi = min(L - 1, (int)ceil(cx + r_out) + 1);
   const int y_lo = max(0, (int)floor(cy - r_out) - 1), y_hi = min(L - 1, (int)ceil(cy + r_out) + 1);
-  const int bw = x_hi - x_lo + 1, bh = y_hi - y_lo + 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool any = x_lo <= x_hi && y_lo <= y_hi;  // (a shift can leave the window)
+  const int tiles = any ? (x_hi - x_lo + 8) >> 3 : 0;  // per row of tiles
   double acc[kSums];
 #pragma unroll
   for (int k = 0; k < kSums; ++k) acc[k] = 0.0;
-  for (int idx = threadIdx.x; idx < bw * bh; idx += blockDim.x) {
-    const int X = x_lo + idx % bw, Y = y_lo + idx / bw;
-    const double ux = X - cx, uy = Y - cy;
-    const double r = sqrt(ux * ux + uy * uy);
-    if (r > r_out) continue;
-    double m = 1.0, dmdr = 0.0;
-    if (r >= r_in) {
-      const double arg = kRefPi * (r - r_in) / (2.0 * g.ehw);
-      m = 0.5 * cos(arg) + 0.5;
-      dmdr = -0.5 * sin(arg) * kRefPi / (2.0 * g.ehw);
+  int tx = warp, ty = 0;
+  for (; any; tx += kGT / 32) {
+    while (tx >= tiles) {
+      tx -= tiles;
+      ++ty;
     }
-    const double x2 = cs * ux + sn * uy + L / 2, y2 = -sn * ux + cs * uy + L / 2;
+    const int X = x_lo + 8 * tx + (lane & 7), Y = y_lo + 4 * ty + (lane >> 3);
+    if (y_lo + 4 * ty > y_hi) break;
+    const double ux = X - cx, uy = Y - cy;
+    const double r2 = ux * ux + uy * uy;
+    if (!(r2 <= out2) || X > x_hi || Y > y_hi) continue;
+    const double xr = cs * ux + sn * uy, yr = cs * uy - sn * ux;
     int k0 = 0, k1 = 0, k2 = 0, k3 = 0;
     double t = 0, u = 0;
     bool inside;
-    bilinear(L, x2, y2, k0, k1, k2, k3, t, u, inside);
-    double R = 0, Rx = 0, Ry = 0, Dv[3] = {0, 0, 0};
-    if (inside) {
-      const double p0 = to_d(P[k0]), p1 = to_d(P[k1]), p2 = to_d(P[k2]), p3 = to_d(P[k3]);
-      R = p0 * (1 - t) * (1 - u) + p1 * t * (1 - u) + p2 * t * u + p3 * (1 - t) * u;
-      Rx = (1 - u) * (p1 - p0) + u * (p2 - p3);
-      Ry = (1 - t) * (p3 - p0) + t * (p2 - p1);
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        const V* Dq = D0 + q * dstride;
-        Dv[q] = to_d(Dq[k0]) * (1 - t) * (1 - u) + to_d(Dq[k1]) * t * (1 - u) + to_d(Dq[k2]) * t * u +
-                to_d(Dq[k3]) * (1 - t) * u;
-      }
-    }
-    const double a = m * R;
-    const double drx = r > 0 ? -ux / r : 0.0, dry = r > 0 ? -uy / r : 0.0;
-    double da[6];
-    da[0] = dmdr * drx * R + m * (Rx * (-cs) + Ry * sn);
-    da[1] = dmdr * dry * R + m * (Rx * (-sn) + Ry * (-cs));
-    da[2] = m * (Rx * (-sn * ux + cs * uy) + Ry * (-cs * ux - sn * uy)) * (kRefPi / 180.0);
-    da[3] = m * Dv[0];
-    da[4] = m * Dv[1];
-    da[5] = m * Dv[2];
+    bilinear(L, xr + L / 2, yr + L / 2, k0, k1, k2, k3, t, u, inside);
     // window sample at the circularly shifted position (zero lag at L/2)
     const int wxl = (X + pk.px + L / 2) & (L - 1), wyl = (Y + pk.py + L / 2) & (L - 1);
     const int ix = wx0 + wxl, iy = wy0 + wyl;
     const double w = (ix < g.nx && iy < g.ny) ? (double)g.img[(size_t)iy * g.nx + ix] * wscale : 0.0;
+    double a = 0, Rx = 0, Ry = 0, da[6] = {0, 0, 0, 0, 0, 0};
+    if (inside) {
+      const float4 p0 = GP::load(P + k0), p1 = GP::load(P + k1), p2 = GP::load(P + k2), p3 = GP::load(P + k3);
+      const double t1 = 1 - t, u1 = 1 - u;
+      const double w0 = t1 * u1, w1 = t * u1, w2 = t * u, w3 = t1 * u;
+      auto mix = [&](float a0, float a1, float a2, float a3) {
+        return (double)a0 * w0 + (double)a1 * w1 + (double)a2 * w2 + (double)a3 * w3;
+      };
+      a = mix(p0.x, p1.x, p2.x, p3.x);
+      Rx = u1 * ((double)p1.x - (double)p0.x) + u * ((double)p2.x - (double)p3.x);
+      Ry = t1 * ((double)p3.x - (double)p0.x) + t * ((double)p2.x - (double)p1.x);
+      da[3] = mix(p0.y, p1.y, p2.y, p3.y);
+      da[4] = mix(p0.z, p1.z, p2.z, p3.z);
+      da[5] = mix(p0.w, p1.w, p2.w, p3.w);
+    }
+    if (r2 >= in2) {  // the mask's soft edge
+      const double r = sqrt(r2);
+      double s, c;
+      sincos(karg * (r - r_in), &s, &c);
+      const double m = 0.5 * c + 0.5;
+      const double q = r > 0 ? 0.5 * s * karg * a / r : 0.0;  // -dm/dr R / r
+      da[0] = q * ux;
+      da[1] = q * uy;
+      a *= m;
+      Rx *= m;
+      Ry *= m;
+      da[3] *= m;
+      da[4] *= m;
+      da[5] *= m;
+    }
+    da[0] += Ry * sn - Rx * cs;
+    da[1] -= Rx * sn + Ry * cs;
+    da[2] = Rx * yr - Ry * xr;  // (per radian: scaled once below)
     acc[0] += a;
     acc[1] += a * a;
     acc[2] += w * a;
@@ -267,7 +320,6 @@ __global__ void __launch_bounds__(kGT) score_grad_kernel(GradArgs g, const V* __
       acc[15 + q] += w * da[q];
     }
   }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int k = 0; k < kSums; ++k) {
     double v = acc[k];
@@ -275,26 +327,36 @@ __global__ void __launch_bounds__(kGT) score_grad_kernel(GradArgs g, const V* __
     if (lane == 0) sh[k][warp] = v;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double S[kSums];
-    for (int k = 0; k < kSums; ++k) {
-      S[k] = 0;
-      for (int w = 0; w < kGT / 32; ++w) S[k] += sh[k][w];
+  if (warp != 0) return;
+  if (lane < kSums) {
+    double v = 0;
+    for (int w = 0; w < kGT / 32; ++w) v += sh[lane][w];
+    if (lane == 5 || lane == 11 || lane == 17) v *= kRefPi / 180.0;
+    sh[lane][0] = v;
+  }
+  __syncwarp();
+  if (lane < 7) {
+    double S[3], D[3];
+    const int q = max(lane - 1, 0);
+    for (int k = 0; k < 3; ++k) {
+      S[k] = sh[k][0];
+      D[k] = sh[3 + 6 * k + q][0];
     }
     const double Sw = g.win_sum[pk.b];
     const double mean = S[0] / L2, var = S[1] / L2 - mean * mean, sd = sqrt(var);
     const double num = S[2] - mean * Sw;
-    const double c = num / (L2 * sd);
     const float2 ms = g.musig[(size_t)pk.b * L * L + (size_t)pk.py * L + pk.px];
-    float* o = out + (size_t)blockIdx.x * 7;
-    o[0] = (float)((c - ms.x) * ms.y);
-    for (int q = 0; q < 6; ++q) {
-      const double dmean = S[3 + q] / L2;
-      const double dvar = 2.0 * S[9 + q] / L2 - 2.0 * mean * dmean;
+    float* o = out + (size_t)blockIdx.x * 7 + lane;
+    if (lane == 0) {
+      const double c = num / (L2 * sd);
+      *o = (float)((c - ms.x) * ms.y);
+    } else {
+      const double dmean = D[0] / L2;
+      const double dvar = 2.0 * D[1] / L2 - 2.0 * mean * dmean;
       const double dsd = dvar / (2.0 * sd);
-      const double dnum = S[15 + q] - dmean * Sw;
+      const double dnum = D[2] - dmean * Sw;
       const double dc = (dnum * sd - num * dsd) / (L2 * sd * sd);
-      o[1 + q] = (float)(dc * ms.y);
+      *o = (float)(dc * ms.y);
     }
   }
 }
@@ -320,23 +382,23 @@ void window_sums(const float* img, int nx, int ny, const int* offx, const int* o
   GISSPA_LAUNCH_CHECK();
 }
 
-void round_templates(const float* prep, long long n1, const float* dprep, long long n2, int precision,
-                     unsigned* absmax, void* out1, void* out2, cudaStream_t s) {
+void grad_plane(const float* in, long long n, int plane, float* table, cudaStream_t s) {
+  plane_kernel<<<ceil_div(n, 256), 256, 0, s>>>(in, n, table + plane);
+  GISSPA_LAUNCH_CHECK();
+}
+void grad_plane(const float2* in, long long n, int plane, float* table, cudaStream_t s) {
+  plane_kernel<<<ceil_div(n, 256), 256, 0, s>>>(in, n, table + plane);
+  GISSPA_LAUNCH_CHECK();
+}
+
+void round_table(const float* table, long long n, int precision, unsigned* absmax, void* out, cudaStream_t s) {
   if (precision == GISSPA_SPEC_FP16) {
     GISSPA_CUDA(cudaMemsetAsync(absmax, 0, sizeof(unsigned), s));
-    abs_max_kernel<<<4 * 148, 256, 0, s>>>(prep, n1, absmax);
+    abs_max_kernel<<<4 * 148, 256, 0, s>>>(table, n, absmax);
     GISSPA_LAUNCH_CHECK();
-    abs_max_kernel<<<4 * 148, 256, 0, s>>>(dprep, n2, absmax);
-    GISSPA_LAUNCH_CHECK();
-    round_kernel<__half><<<ceil_div(n1, 256), 256, 0, s>>>(prep, n1, absmax, static_cast<__half*>(out1));
-    GISSPA_LAUNCH_CHECK();
-    round_kernel<__half><<<ceil_div(n2, 256), 256, 0, s>>>(dprep, n2, absmax, static_cast<__half*>(out2));
+    round_kernel<__half><<<ceil_div(n, 256), 256, 0, s>>>(table, n, absmax, static_cast<__half*>(out));
   } else {
-    round_kernel<__nv_bfloat16><<<ceil_div(n1, 256), 256, 0, s>>>(prep, n1, nullptr,
-                                                                  static_cast<__nv_bfloat16*>(out1));
-    GISSPA_LAUNCH_CHECK();
-    round_kernel<__nv_bfloat16><<<ceil_div(n2, 256), 256, 0, s>>>(dprep, n2, nullptr,
-                                                                  static_cast<__nv_bfloat16*>(out2));
+    round_kernel<__nv_bfloat16><<<ceil_div(n, 256), 256, 0, s>>>(table, n, nullptr, static_cast<__nv_bfloat16*>(out));
   }
   GISSPA_LAUNCH_CHECK();
 }
@@ -344,13 +406,11 @@ void round_templates(const float* prep, long long n1, const float* dprep, long l
 void score_grads(const GradArgs& g, const GradPick* picks, int n, float* out, cudaStream_t s) {
   if (n <= 0) return;
   if (g.precision == GISSPA_SPEC_FP16)
-    score_grad_kernel<__half><<<n, kGT, 0, s>>>(g, static_cast<const __half*>(g.prep_lp),
-                                                 static_cast<const __half*>(g.dprep_lp), picks, out);
+    score_grad_kernel<__half><<<n, kGT, 0, s>>>(g, picks, out);
   else if (g.precision == GISSPA_SPEC_BF16)
-    score_grad_kernel<__nv_bfloat16><<<n, kGT, 0, s>>>(g, static_cast<const __nv_bfloat16*>(g.prep_lp),
-                                                        static_cast<const __nv_bfloat16*>(g.dprep_lp), picks, out);
+    score_grad_kernel<__nv_bfloat16><<<n, kGT, 0, s>>>(g, picks, out);
   else
-    score_grad_kernel<float><<<n, kGT, 0, s>>>(g, g.prep, g.dprep, picks, out);
+    score_grad_kernel<float><<<n, kGT, 0, s>>>(g, picks, out);
   GISSPA_LAUNCH_CHECK();
 }
 

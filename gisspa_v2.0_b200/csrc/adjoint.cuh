@@ -13,12 +13,9 @@ struct GradPick {
 };
 
 struct GradArgs {
-  const float* prep;       // [nt][L][L] prepared templates (real space) at the CTF evaluated
-  const float* dprep;      // [3][nt][L][L] d prep / d(dfu, dfv, dfang)
-  // The same two arrays stored in the handle's template precision (GISSPA_SPEC_FP16 / BF16:
-  // 2-byte values read in place of prep / dprep); precision GISSPA_SPEC_FP32 reads the above.
-  const void* prep_lp;
-  const void* dprep_lp;
+  // [nt][L][L][4]: the prepared template (real space) at the CTF evaluated and its derivatives
+  // by dfu, dfv and dfang; float, or __half / __nv_bfloat16 at that template precision
+  const void* table;
   int precision;
   const float* img;        // [ny][nx] preprocessed micrograph
   int nx, ny;
@@ -39,11 +36,12 @@ void scale_by_table(const float2* F, const float* tab, const double* m, int nt, 
 // work: reduce_bytes(l, nwin)
 void window_sums(const float* img, int nx, int ny, const int* offx, const int* offy, int bx, int nwin, int l,
                  const double* win_m, double* out, double* work, cudaStream_t s);
-// prep (n1 values) and dprep (n2) rounded to the template precision (1: FP16, 2: BF16) into out1,
-// out2; FP16 first scales both by one power of two that fits their largest value (absmax: one
-// unsigned of device scratch)
-void round_templates(const float* prep, long long n1, const float* dprep, long long n2, int precision,
-                     unsigned* absmax, void* out1, void* out2, cudaStream_t s);
+// Entry `plane` of the table's pixels, from real images or the real parts of complex ones
+void grad_plane(const float* in, long long n, int plane, float* table, cudaStream_t s);
+void grad_plane(const float2* in, long long n, int plane, float* table, cudaStream_t s);
+// The table's n values rounded to the template precision (1: FP16, 2: BF16); FP16 first scales them
+// by one power of two that fits the largest (absmax: one unsigned of device scratch)
+void round_table(const float* table, long long n, int precision, unsigned* absmax, void* out, cudaStream_t s);
 // out: n x 7 floats (z, dz/d(dx, dy, theta, dfu, dfv, dfang))
 void score_grads(const GradArgs& g, const GradPick* picks, int n, float* out, cudaStream_t s);
 

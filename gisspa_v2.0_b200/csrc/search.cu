@@ -1592,13 +1592,15 @@ void adjoint_prepare(gisspa_handle* h, const gisspa_ctf& ctf) {
   h->keep_whitened = false;
   float* dtab = buf<float>(h->dtab, 3 * (size_t)c.L2);
   ctf_dweight(dtab, l, c.p, c.s);
-  float* dprep = buf<float>(h->dprep, 3 * (size_t)nt * c.L2);
+  const long long n = (long long)nt * c.L2;
+  float* table = buf<float>(h->grad_tab, 4 * (size_t)n);
+  grad_plane(h->prep_real.as<float>(), n, 0, table, c.s);
   float2* tb = buf<float2>(h->tb, (size_t)nt * c.L2);
   float2* tmp = buf<float2>(h->tb_tmp, (size_t)nt * c.L2);
   for (int q = 0; q < 3; ++q) {
     scale_by_table(h->tw_spec.as<float2>(), dtab + (size_t)q * c.L2, h->tmpl_m.as<double>(), nt, l, tb, c.s);
     h->fft.fft2(tb, tmp, nt, l, l, +1, 1.f, c.s);  // same unnormalised IFFT as the prepared templates
-    real_part(tb, dprep + (size_t)q * nt * c.L2, (long long)nt * c.L2, 1.f, c.s);
+    grad_plane(tb, n, 1 + q, table, c.s);
   }
   window_sums(h->img_pre.as<float>(), h->last_nx, h->last_ny, h->offx.as<int>(), h->offy.as<int>(), h->last_bx,
               h->last_W, l, h->win_m.as<double>(), buf<double>(h->win_sum, h->last_W),
@@ -1606,19 +1608,14 @@ void adjoint_prepare(gisspa_handle* h, const gisspa_ctf& ctf) {
   // the FP16 / BF16 template forms evaluate from templates stored at that precision
   const int prec = h->cfg.spectrum_precision;
   if (prec != GISSPA_SPEC_FP32)
-    round_templates(h->prep_real.as<float>(), (long long)nt * c.L2, dprep, 3LL * nt * c.L2, prec,
-                    buf<unsigned>(h->lp_scale, 1), buf<__half>(h->prep_lp, (size_t)nt * c.L2),
-                    buf<__half>(h->dprep_lp, 3 * (size_t)nt * c.L2), c.s);
+    round_table(table, 4 * n, prec, buf<unsigned>(h->lp_scale, 1), buf<__half>(h->grad_lp, 4 * (size_t)n), c.s);
 }
 
 void eval_grads(gisspa_handle* h, const std::vector<GradPick>& gp, std::vector<float>& out) {
   const int n = (int)gp.size();
   GradArgs g{};
-  g.prep = h->prep_real.as<float>();
-  g.dprep = h->dprep.as<float>();
   g.precision = h->cfg.spectrum_precision;
-  g.prep_lp = g.precision != GISSPA_SPEC_FP32 ? h->prep_lp.as<void>() : nullptr;
-  g.dprep_lp = g.precision != GISSPA_SPEC_FP32 ? h->dprep_lp.as<void>() : nullptr;
+  g.table = g.precision != GISSPA_SPEC_FP32 ? h->grad_lp.as<void>() : h->grad_tab.as<void>();
   g.img = h->img_pre.as<float>();
   g.nx = h->last_nx;
   g.ny = h->last_ny;
