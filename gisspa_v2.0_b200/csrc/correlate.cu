@@ -364,11 +364,6 @@ __global__ void __launch_bounds__(NW * 32, MINB)
             }
           }
         }
-      } else if constexpr (EPI == EPI_MAP) {
-        float* out = a.map_out + (size_t)p * L * L + (size_t)oy * L;
-#pragma unroll
-        for (int i = 0; i < E; ++i)
-          *reinterpret_cast<float2*>(out + ox[i]) = make_float2(v[i].x * inv, v[i].y * inv);
       }
     }
     if constexpr (EPI == EPI_CHUNK && L % 256 != 0) {
@@ -442,6 +437,62 @@ void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaSt
   cfg.numAttrs = 1;
   GISSPA_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
   ++launch_counter();
+}
+
+constexpr int kMapGroups = 148 * 16;  // CTAs of one row per team below which a launch keeps them
+// Pass B of EPI_MAP: the pairs of a launch are independent (nothing is summed over templates), so
+// every row of every pair is a team's own work: teams load their rows themselves, without the bulk
+// copies and their bounded waits.  `per` rows per team share the CTA's tables.
+template <int L>
+struct MapShape {
+  static constexpr int TEAM = L <= 320 ? 16 : 32, NW = L <= 320 ? 4 : 8, NTEAM = NW * 32 / TEAM;
+};
+template <int L>
+__global__ void __launch_bounds__(MapShape<L>::NW * 32)
+    map_rows_kernel(CorrArgs a, int per, const float2* __restrict__ twL, const float2* __restrict__ twNZ) {
+  using S = MapShape<L>;
+  using RX = RowXform<L, S::TEAM>;
+  constexpr int NZ = L / 2, TEAM = S::TEAM, NV = NZ / 2 / TEAM;
+  static_assert(NZ / 2 % TEAM == 0, "16-byte loads split evenly over a team");
+  __shared__ __align__(16) float2 rows[S::NTEAM][NZ];
+  __shared__ __align__(16) float2 tw_nz[NZ + NZ / 16], tw_l[NZ];
+  griddep_launch_dependents();
+  for (int i = threadIdx.x; i < NZ; i += S::NW * 32) {
+    tw_nz[tw_pad_index(i)] = __ldg(twNZ + i);
+    tw_l[i] = __ldg(twL + i);
+  }
+  __syncthreads();
+  const int team = threadIdx.x / TEAM, lt = threadIdx.x - team * TEAM;
+  const int p = blockIdx.y, e = p / a.D, d = p - e * a.D;
+  const float inv = 1.0f / (float)(L * L);
+  float2* row = rows[team];
+  float* map = a.map_out + ((size_t)e * a.nt_total + a.n0 + d) * L * L;
+  griddep_wait();  // Q comes from the pass A just before
+  for (int q = 0; q < per; ++q) {
+    const int y = (blockIdx.x * per + q) * S::NTEAM + team;
+    const float4* src = reinterpret_cast<const float4*>(a.Q + ((size_t)p * L + y) * NZ);
+    float4 in[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) in[i] = src[lt + i * TEAM];
+    __syncwarp();  // the row before has been read
+#pragma unroll
+    for (int i = 0; i < NV; ++i) reinterpret_cast<float4*>(row)[lt + i * TEAM] = in[i];
+    __syncwarp();
+    float2 v[RX::EBUF];
+    RX::run(v, row, tw_nz, tw_l, lt, WarpSync{});
+    float* out = map + (size_t)((y + L / 2) % L) * L;
+#pragma unroll
+    for (int i = 0; i < RX::EOUT; ++i)
+      __stcs(reinterpret_cast<float2*>(out + (2 * RX::out_index(lt, i) + L / 2) % L),
+             make_float2(v[i].x * inv, v[i].y * inv));
+  }
+}
+template <int L>
+void launch_map(const CorrLaunch& cl, const CorrArgs& args, const float2* twL, const float2* twNZ, cudaStream_t s) {
+  constexpr int G = L / MapShape<L>::NTEAM;  // row groups per pair
+  const int per = (long long)cl.D * cl.E * G >= kMapGroups ? 4 : 1;
+  static_assert(G % 4 == 0, "whole CTAs per pair");
+  launch_pdl(map_rows_kernel<L>, dim3(G / per, cl.D * cl.E), dim3(MapShape<L>::NW * 32), 0, s, args, per, twL, twNZ);
 }
 
 // Pass A's mask: pairs only where pass B lists the live templates (D small enough).
@@ -537,7 +588,6 @@ void launch_b(const CorrLaunch& cl, const CorrArgs& args, const float2* twL, con
       case EPI_SUMMAX: launch_b_cfg<L, P::TEAM, P::RB, P::NW, EPI_SUMMAX, P::MINB>(cl, args, twL, twNZ, s); break;
       case EPI_TOPK: launch_b_cfg<L, P::TEAM, P::RB, P::NW, EPI_TOPK, P::MINB>(cl, args, twL, twNZ, s); break;
       case EPI_CHUNK: launch_b_cfg<L, P::TEAM, P::RB, P::NW, EPI_CHUNK, P::MINB>(cl, args, twL, twNZ, s); break;
-      case EPI_MAP: launch_b_cfg<L, P::TEAM, P::RB, P::NW, EPI_MAP, P::MINB>(cl, args, twL, twNZ, s); break;
       default: throw CudaError{cudaErrorInvalidValue, "pass B shape without this epilogue"};
     }
     return;
@@ -548,7 +598,6 @@ void launch_b(const CorrLaunch& cl, const CorrArgs& args, const float2* twL, con
     case EPI_CHUNK: launch_b_cfg<L, P::TEAM, P::RB, P::NW, EPI_CHUNK, P::MINB>(cl, args, twL, twNZ, s); break;
     case EPI_TOPK: launch_b_cfg<L, P::TEAM, P::RB, P::NW, EPI_TOPK, P::MINB>(cl, args, twL, twNZ, s); break;
     case EPI_NONORM: launch_b_cfg<L, P::TEAM, P::RB, P::NW, EPI_NONORM, P::MINB>(cl, args, twL, twNZ, s); break;
-    case EPI_MAP: launch_b_cfg<L, P::TEAM, P::RB, P::NW, EPI_MAP, P::MINB>(cl, args, twL, twNZ, s); break;
     default: throw CudaError{cudaErrorInvalidValue, "unknown epilogue"};
   }
   }
@@ -570,6 +619,11 @@ int launch_pair(const CorrLaunch& cl, const float2* I, const void* T, float2* Q,
     default: throw CudaError{cudaErrorInvalidValue, "unknown spectrum precision"};
   }
   if (ev) GISSPA_CUDA(cudaEventRecord(ev[1], s));
+  if (cl.epi == EPI_MAP) {
+    launch_map<L>(cl, args, twL, twNZ, s);
+    if (ev) GISSPA_CUDA(cudaEventRecord(ev[2], s));
+    return 2;
+  }
   if constexpr (L == 512) {
     if (cl.tc && cl.spec == GISSPA_SPEC_FP16 && cl.epi == EPI_TOPK) {
       launch_b_tc(cl, args, twL, twNZ, s);
@@ -622,7 +676,7 @@ bool correlate_variant_ok(int L, int variant, int epi) {
   if (variant < 0 || variant >= correlate_variants(L)) return false;
   if (variant == engine_variant(L)) return engine_supported(L, epi);
   const bool wide = L == 1024 && variant >= 3;  // 64-lane rows
-  return !wide || epi == EPI_SUM || epi == EPI_SUMMAX || epi == EPI_TOPK || epi == EPI_CHUNK || epi == EPI_MAP;
+  return !wide || epi == EPI_SUM || epi == EPI_SUMMAX || epi == EPI_TOPK || epi == EPI_CHUNK;
 }
 
 int correlate_launch(const CorrLaunch& cl, const float2* I, const void* T, float2* Q, const CorrArgs& args_in,

@@ -101,7 +101,7 @@ struct CorrArgs {
   unsigned long long* nn_key;
   double* nn_sum;           // [W][nt_total][2]
   float border;             // diameter / 4
-  // EPI_MAP, [pairs][L][L]
+  // EPI_MAP, [window of the launch][nt_total][L][L]
   float* map_out;
 };
 

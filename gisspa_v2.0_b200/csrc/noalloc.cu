@@ -26,9 +26,6 @@ static __device__ __align__(256) float2 g_noalloc_scratch[kNoAllocScratchBytes /
 // Twiddle tables exp(-2 pi i p / n) for n = 1024, 512, 256, 128, back to back.
 constexpr int kTwTotal = 1024 + 512 + 256 + 128;
 static __device__ __align__(256) float2 g_noalloc_twiddles[kTwTotal];
-// Set by a kernel whose bounded wait gave up.  Every call zeroes it on its stream before
-// its launches and reads it back after them.
-static __device__ unsigned g_noalloc_flag;
 
 int tw_offset(int n) { return n == 1024 ? 0 : n == 512 ? 1024 : n == 256 ? 1536 : 1792; }
 
@@ -36,7 +33,6 @@ struct DeviceSlot {
   bool ready = false;
   float2* scratch = nullptr;
   float2* twiddles = nullptr;
-  unsigned* flag = nullptr;
 };
 std::mutex g_mu;
 DeviceSlot g_slots[64];
@@ -61,12 +57,6 @@ int setup(int dev, std::string& err) {
     return GISSPA_ERR_CUDA;
   }
   s.twiddles = static_cast<float2*>(p);
-  e = cudaGetSymbolAddress(&p, g_noalloc_flag);
-  if (e != cudaSuccess) {
-    err = std::string("cudaGetSymbolAddress(flag): ") + cudaGetErrorString(e);
-    return GISSPA_ERR_CUDA;
-  }
-  s.flag = static_cast<unsigned*>(p);
   float2 h[kTwTotal];
   for (int n : {1024, 512, 256, 128})
     for (int k = 0; k < n; ++k) {
@@ -130,24 +120,12 @@ static int cc_maps_noalloc(const void* d_windows, int n_windows, const void* d_t
   args.nt_real = n_templates;
   args.nt_total = n_templates;
   args.map_out = d_out;
-  args.err = ds.flag;
   CorrLaunch cl{L, n_windows, n_templates, spec, EPI_MAP, 0};
   const cudaStream_t cs = static_cast<cudaStream_t>(stream);
   try {
-    // The flag keeps the previous call's value: clear it on this call's stream first.
-    GISSPA_CUDA(cudaMemsetAsync(ds.flag, 0, sizeof(unsigned), cs));
     correlate_launch(cl, static_cast<const float2*>(d_windows), d_templates, ds.scratch, args,
                      ds.twiddles + tw_offset(L), ds.twiddles + tw_offset(L / 2), cs);
-    // A row kernel whose bounded wait for its slice of the intermediate gave up leaves its
-    // maps partly unwritten: wait for the launches and report that as a timeout.
     GISSPA_CUDA(cudaStreamSynchronize(cs));
-    unsigned flag = 0;
-    GISSPA_CUDA(cudaMemcpy(&flag, ds.flag, sizeof(flag), cudaMemcpyDeviceToHost));
-    if (flag) {
-      err = "cc_maps_noalloc: a bounded wait inside the correlation kernels gave up (GPU overloaded or "
-            "stalled); the maps are incomplete";
-      return GISSPA_ERR_TIMEOUT;
-    }
   } catch (const CudaError& ce) {
     err = std::string(cudaGetErrorString(ce.code)) + " at " + ce.where;
     return GISSPA_ERR_CUDA;

@@ -1757,39 +1757,49 @@ void refine_run(gisspa_handle* h, gisspa_pick* picks, size_t n, int steps, gissp
   if (ctf) *ctf = ctf_of(psi);
 }
 
+// All windows and a few templates per launch, as many pairs as keep their intermediate in L2
+// beside the spectra: with every template of one window per launch, 24 pairs of window 1024 wrote
+// and read 100 MB of it through DRAM.
+constexpr size_t kMapBatchBytes = 32u << 20;
 void cc_maps(gisspa_handle* h, const void* d_win, int nw, const void* d_t, int ntm, int spec, float* d_out) {
   Ctx c{h, h->stream, h->cfg.window_size, (long long)h->cfg.window_size * h->cfg.window_size, DevParams{}};
   const int l = c.l;
   CorrArgs args{};
-  args.map_out = d_out;
   args.nt_real = ntm;
   args.nt_total = ntm;
-  args.err = buf<unsigned>(h->dev_err, 1);
-  GISSPA_CUDA(cudaMemsetAsync(args.err, 0, sizeof(unsigned), c.s));
-  const bool generic = !correlate_fast(l);
-  float2* Q = generic ? nullptr : buf<float2>(h->Q, (size_t)ntm * (l / 2) * l);
-  const float2* twL = generic ? nullptr : h->fft.twiddles(l);
-  const float2* twNZ = generic ? nullptr : h->fft.twiddles(l / 2);
-  float2* gz = generic ? buf<float2>(h->gen_z, generic_z_elems(l, ntm)) : nullptr;
-  const size_t xe = generic ? generic_x_elems(l, ntm, EPI_MAP) : 0;
-  float2* gx = xe ? buf<float2>(h->gen_x, xe) : nullptr;
-  // one launch per window: pair p = d covers template d of window b, written at [b][d]
-  for (int b = 0; b < nw; ++b) {
-    CorrLaunch cl{l, 1, ntm, spec, EPI_MAP};
-    args.Q = Q;
-    args.b0 = b;
-    args.n0 = 0;
+  if (!correlate_fast(l)) {
+    float2* gz = buf<float2>(h->gen_z, generic_z_elems(l, ntm));
+    const size_t xe = generic_x_elems(l, ntm, EPI_MAP);
+    float2* gx = xe ? buf<float2>(h->gen_x, xe) : nullptr;
     args.D = ntm;
+    for (int b = 0; b < nw; ++b) {
+      args.b0 = b;
+      args.map_out = d_out + (size_t)b * ntm * c.L2;
+      correlate_generic(CorrLaunch{l, 1, ntm, spec, EPI_MAP}, static_cast<const float2*>(d_win), d_t, args, h->fft, gz,
+                        gx, c.s);
+    }
+    GISSPA_CUDA(cudaStreamSynchronize(c.s));
+    return;
+  }
+  const size_t per = (size_t)(l / 2) * l;
+  const int P = std::max(1, (int)(kMapBatchBytes / (per * sizeof(float2))));
+  const int E = std::min(nw, P), D = std::min(ntm, std::max(1, P / E));
+  float2* Q = buf<float2>(h->Q, per * E * D);
+  args.Q = Q;
+  CorrLaunch cl{l, E, D, spec, EPI_MAP};
+  for (int b = 0; b < nw; b += E) {
+    cl.E = std::min(E, nw - b);
+    args.b0 = b;
     args.map_out = d_out + (size_t)b * ntm * c.L2;
-    if (generic)
-      correlate_generic(cl, static_cast<const float2*>(d_win), d_t, args, h->fft, gz, gx, c.s);
-    else
-      correlate_launch(cl, static_cast<const float2*>(d_win), d_t, Q, args, twL, twNZ, c.s);
+    for (int t = 0; t < ntm; t += D) {
+      cl.D = args.D = std::min(D, ntm - t);
+      args.n0 = t;
+      correlate_launch(cl, static_cast<const float2*>(d_win), d_t, Q, args, h->fft.twiddles(l),
+                       h->fft.twiddles(l / 2), c.s);
+      cl.chained = true;
+    }
   }
   GISSPA_CUDA(cudaStreamSynchronize(c.s));
-  unsigned flag = 0;
-  GISSPA_CUDA(cudaMemcpy(&flag, args.err, sizeof(flag), cudaMemcpyDeviceToHost));
-  if (flag) throw TimeoutError{"cc_maps"};
 }
 
 void project_run(gisspa_handle* h, const float* volume, int nx, int ny, int nz, const float* angles, int n, int ri,

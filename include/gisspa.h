@@ -260,13 +260,11 @@ int gisspa_cc_maps(gisspa_handle* h, const void* d_windows, int n_windows, const
  * GISSPA_ERR_CAPACITY with the reason in gisspa_last_error(NULL).  d_windows,
  * d_templates, d_out and window_size as for gisspa_cc_maps; runs on `stream`
  * (a cudaStream_t, NULL = default stream) of the current device and returns once the
- * maps are written (it waits for `stream`).  GISSPA_ERR_TIMEOUT: a bounded wait inside
- * the kernels gave up and the maps are incomplete (the next call starts clean).  The
- * first call on each device sets up that device's copy of the arrays (make that first
- * call before any stream capture).  Every call shares the one intermediate and error
- * flag, which keep the last call's contents; the intermediate is fully overwritten
- * before it is read and the flag is cleared at the start of each call, so calls that
- * overlap on the GPU (other streams or threads) race on them and must be serialised by
+ * maps are written (it waits for `stream`).  The first call on each device sets up that
+ * device's copy of the arrays (make that first call before any stream capture).  Every
+ * call shares the one intermediate, which keeps the last call's contents and is fully
+ * overwritten before it is read, so calls that
+ * overlap on the GPU (other streams or threads) race on it and must be serialised by
  * the caller. */
 int gisspa_cc_maps_noalloc(const void* d_windows, int n_windows, const void* d_templates, int n_templates,
                            int window_size, int spec, float* d_out, void* stream);
