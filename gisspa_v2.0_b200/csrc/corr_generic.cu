@@ -1,6 +1,6 @@
 // corr_generic.cu — the correlation and its epilogues for window sizes without hand-tuned
 // kernels.  Same results as pass A + pass B (correlate.cu) within FP32 rounding: the
-// transforms run in shared memory (mixed radix 2/3/4/5/7) in a fused two-pass form, or on the
+// transforms run in shared memory (mixed radix, fft_smooth.cuh) in a fused two-pass form, or on the
 // generic FFT engine (Bluestein for other lengths) in an unfused form; the epilogues reproduce
 // pass B's per-pixel sums and maxima, chunk picks with the reference's tie order, norm_type=0
 // peaks and sums, and maps.  The reference's chunks are 256 consecutive pixels of the window's
@@ -181,6 +181,11 @@ __global__ void gen_map_kernel(const float2* __restrict__ X, CorrArgs a, int L) 
 }
 
 // ---- fused two-pass form for window sizes whose prime factors are 2, 3, 5 and 7
+// Both passes are bound by instruction issue and shared memory.  Stages of 2 to 16 points in
+// registers (336 = 7 6 8) instead of 2, 3, 4, 5 and 7 with table reads per point, multiplications
+// instead of divisions by run-time sizes, rows per CTA that fill its passes, and an intermediate
+// that both passes move in whole sectors took a top-K search of 1500 x 1401 pixels at window 336
+// (20 templates, 30 angles) from 59.1 to 35.0 ms.
 
 // Rows per CTA of gen_rows_kernel: even, a divisor of L, about 1280 pixels per CTA, and for
 // the chunk scans (EPI_CHUNK, EPI_NONORM) RB L a multiple of 256; 0 when no such RB exists.
@@ -199,32 +204,51 @@ __host__ __device__ constexpr int gen_rows_rb(int L, int epi) {
 }
 
 
+// Where the column pass leaves Z[p][kx][y]: four rows of a column together (L is a multiple of 16),
+// the columns side by side, so that both passes move whole 32-byte sectors: from [kx][y] the row
+// pass read 16 bytes of a sector per column, twice.
+__device__ __forceinline__ size_t gen_z_index(int p, int kx, int y, int L, int hz) {
+  return (((size_t)p * (L >> 2) + (y >> 2)) * hz + kx) * 4 + (y & 3);
+}
+constexpr int kGenColPad = 4;  // the columns' stride in shared memory, beyond L: writes without bank conflicts
+
 // Column pass: rows gr = p (L/2+1) + kx of the launch's half-spectrum products
 // I[b0 + e][kx][.] conj(T[n0 + d][kx][.]) (p = e D + d), each inverse-transformed along ky in
-// shared memory: Z[p][kx][y].
-template <int LC, typename SPEC>
-__global__ void gen_cols_kernel(const float2* __restrict__ I, const typename SPEC::T* __restrict__ T, int b0, int n0,
-                                int D, int L_, long long nrows, int rpc, SmoothPlan plan, const float2* __restrict__ tw,
-                                float2* __restrict__ Z) {
+// shared memory: Z (gen_z_index).  rpc <= kGenMaxCols
+constexpr int kGenMaxCols = 128;
+template <typename SPEC>
+__global__ void __launch_bounds__(256) gen_cols_kernel(const float2* __restrict__ I,
+                                                       const typename SPEC::T* __restrict__ T, int b0, int n0, int D,
+                                                       int L, unsigned div_l, int nrows, int rpc, SmoothPlan plan,
+                                                       const float2* __restrict__ tw, float2* __restrict__ Z) {
   extern __shared__ float2 sm[];
-  const int L = LC ? LC : L_;
-  const int hz = L / 2 + 1;
+  __shared__ long long iof[kGenMaxCols], tof[kGenMaxCols];
+  __shared__ int zp[kGenMaxCols], zk[kGenMaxCols];
+  const int hz = L / 2 + 1, ld = L + kGenColPad;
   const long long H = (long long)hz * L;
-  const long long row0 = (long long)blockIdx.x * rpc;
-  const int rows_here = (int)min((long long)rpc, nrows - row0);
+  const int row0 = blockIdx.x * rpc;
+  const int rows_here = min(rpc, nrows - row0);
   float2* a = sm;
-  float2* b = sm + (size_t)rpc * L;
-  for (int i = threadIdx.x; i < rows_here * L; i += blockDim.x) {
-    const int r = i / L, k = i - r * L;
-    const long long gr = row0 + r;
-    const int p = (int)(gr / hz), kx = (int)(gr - (long long)p * hz);
-    const int e = p / D, d = p - e * D;
-    a[i] = cmulc(I[(size_t)(b0 + e) * H + (size_t)kx * L + k],
-                 SPEC::load(T + (size_t)(n0 + d) * H + (size_t)kx * L + k));
+  float2* b = sm + (size_t)rpc * ld;
+  for (int r = threadIdx.x; r < rows_here; r += 256) {
+    const int gr = row0 + r, p = gr / hz, kx = gr - p * hz, e = p / D, d = p - e * D;
+    iof[r] = (b0 + e) * H + (long long)kx * L;
+    tof[r] = (n0 + d) * H + (long long)kx * L;
+    zp[r] = p;
+    zk[r] = kx;
   }
   __syncthreads();
-  const float2* f = smooth_stages_l<LC, 1>(a, b, rows_here, L, L, plan, tw);
-  for (int i = threadIdx.x; i < rows_here * L; i += blockDim.x) Z[(size_t)row0 * L + i] = f[i];
+  for (int i = threadIdx.x; i < rows_here * L; i += 256) {
+    const int r = fast_div(i, div_l), k = i - r * L;
+    a[r * ld + k] = cmulc(I[iof[r] + k], SPEC::load(T + tof[r] + k));
+  }
+  __syncthreads();
+  const float2* f = smooth_stages<1>(a, b, rows_here, L, ld, plan, tw);
+  const unsigned div_r = fast_div_mul(rows_here);
+  for (int i = threadIdx.x; i < rows_here * L; i += 256) {
+    const int j = i & 3, q = i >> 2, yb = fast_div(q, div_r), r = q - yb * rows_here, y = yb * 4 + j;
+    Z[gen_z_index(zp[r], zk[r], y, L, hz)] = f[r * ld + y];
+  }
 }
 
 // Row pass: one CTA per (block of RB window rows, window of the launch), over the launch's D
@@ -238,24 +262,25 @@ __global__ void gen_cols_kernel(const float2* __restrict__ I, const typename SPE
 // 256-pixel scan and q = 256 i + t is pixel t of the CTA's chunk i.  The rows of up to TB
 // templates go through one transform pass (fewer block barriers, more butterflies per thread);
 // the epilogue then takes those templates in order.
-template <int LC, int EPI>
-__global__ void __launch_bounds__(256) gen_rows_kernel(const float2* __restrict__ Z, CorrArgs a, int L_, int RB_,
-                                                       int TB, SmoothPlan plan, const float2* __restrict__ tw) {
+template <int EPI>
+__global__ void __launch_bounds__(256, 3) gen_rows_kernel(const float2* __restrict__ Z, CorrArgs a, int L, unsigned div_l,
+                                                       int RB, int ld, int TB, SmoothPlan plan,
+                                                       const float2* __restrict__ tw) {
   extern __shared__ float2 sm[];
-  constexpr int kRB = LC ? gen_rows_rb(LC, EPI) : 0;
-  static_assert(LC == 0 || kRB > 0, "no row block for LC");
-  const int L = LC ? LC : L_, RB = LC ? kRB : RB_, ld = L + 1;
+  const int hz = L / 2 + 1;
   const int hr = RB / 2, npix = RB * L, nch = npix / 256, t = threadIdx.x, lane = t & 31, wid = t >> 5;
   float2* buf0 = sm;  // TB templates x hr complex rows, row stride ld
   float2* buf1 = sm + (size_t)TB * hr * ld;
   unsigned long long* red = reinterpret_cast<unsigned long long*>(sm + (size_t)2 * TB * hr * ld);  // [nch][8]
   double* dred = reinterpret_cast<double*>(red + (size_t)nch * 8);                            // [2][8]
   char* st = reinterpret_cast<char*>(dred + 16);
+  __shared__ unsigned hits;  // EPI_CHUNK: the group's templates with a pixel at the threshold
   const int e = blockIdx.y, win = a.b0 + e, Y0 = blockIdx.x * RB;
-  const long long L2 = (long long)L * L, H = (long long)(L / 2 + 1) * L;
+  const long long L2 = (long long)L * L;
   const size_t wpix = (size_t)win * L2 + (size_t)Y0 * L;
   const float inv = 1.0f / (float)L2;
   const int angle = a.angle_state ? a.angle_state->index : a.angle;
+  const unsigned div_hr = fast_div_mul(hr), div_hz = fast_div_mul(hz);
   float* s1 = reinterpret_cast<float*>(st);  // SUM / TOPK per-pixel accumulators
   float* s2 = s1 + npix;
   float* bst = s2 + npix;
@@ -273,62 +298,87 @@ __global__ void __launch_bounds__(256) gen_rows_kernel(const float2* __restrict_
   }
   if constexpr (EPI == EPI_CHUNK)
     for (int q = t; q < npix; q += 256) ms[q] = a.musig[wpix + q];
+  // pixel q's place in a template's transformed rows (complex row, column) and which part
+  auto place = [&](int q, bool& upper) {
+    const int r = fast_div(q, div_l), ox = q - r * L, x = ox + L / 2 - (ox + L / 2 >= L ? L : 0);
+    upper = r >= hr;
+    return (upper ? r - hr : r) * ld + x;
+  };
 
   for (int d0 = 0; d0 < a.D; d0 += TB) {
     const int nd = min(TB, a.D - d0);
-    for (int idx = t; idx < nd * hr * L; idx += 256) {
-      const int g = idx / (hr * L), rem = idx - g * (hr * L);
-      const int k = rem / hr, r2 = rem - k * hr;
-      const float2* Zp = Z + (size_t)(e * a.D + d0 + g) * H;
-      const int ya = (Y0 + r2 + L / 2) % L, yb = (Y0 + r2 + hr + L / 2) % L;
-      float2 A, B;
-      if (k <= L / 2) {
-        A = Zp[(size_t)k * L + ya];
-        B = Zp[(size_t)k * L + yb];
-      } else {
-        A = Zp[(size_t)(L - k) * L + ya];
-        B = Zp[(size_t)(L - k) * L + yb];
-        A.y = -A.y;
-        B.y = -B.y;
-      }
-      buf0[(size_t)(g * hr + r2) * ld + k] = make_float2(A.x - B.y, A.y + B.x);
+    if (EPI == EPI_CHUNK && t == 0) hits = 0u;
+    for (int idx = t; idx < nd * hr * hz; idx += 256) {
+      const int q = fast_div(idx, div_hr), r2 = idx - q * hr, g = fast_div(q, div_hz), k = q - g * hz;
+      int ya = Y0 + r2 + L / 2, yb = ya + hr;
+      ya -= ya >= L ? L : 0;
+      yb -= yb >= L ? L : 0;
+      const int p = e * a.D + d0 + g;
+      const float2 A = Z[gen_z_index(p, k, ya, L, hz)], B = Z[gen_z_index(p, k, yb, L, hz)];
+      float2* row = buf0 + (g * hr + r2) * ld;
+      row[k] = make_float2(A.x - B.y, A.y + B.x);
+      if (k > 0 && 2 * k < L) row[L - k] = make_float2(A.x + B.y, B.x - A.y);
     }
     __syncthreads();
-    const float2* fg = smooth_stages_l<LC, 1>(buf0, buf1, nd * hr, L, ld, plan, tw);
+    const float2* fg = smooth_stages<1>(buf0, buf1, nd * hr, L, ld, plan, tw);
 
-    // the group's templates in order, so every pixel folds them as the one-at-a-time sweep would
-    for (int g = 0; g < nd; ++g) {
-      const int d = d0 + g, p = e * a.D + d;
-      const float2* f = fg + (size_t)g * hr * ld;
-
-      if constexpr (EPI == EPI_SUM || EPI == EPI_TOPK) {
-        for (int q = t; q < npix; q += 256) {
-          const int r = q / L, ox = q - r * L, x = ox + L / 2 - (ox + L / 2 >= L ? L : 0);
-          const float2 w = f[(size_t)(r < hr ? r : r - hr) * ld + x];
-          const float c = (r < hr ? w.x : w.y) * inv;
-          s1[q] += c;
-          s2[q] = fmaf(c, c, s2[q]);
+    // each pixel folds the group's templates in order, as the one-at-a-time sweep would
+    if constexpr (EPI == EPI_SUM || EPI == EPI_TOPK) {
+      for (int q = t; q < npix; q += 256) {
+        bool up;
+        const float2* f = fg + place(q, up);
+        float v1 = s1[q], v2 = s2[q], b = 0.f;
+        int arg = -1;
+        if constexpr (EPI == EPI_TOPK) b = bst[q];
+        for (int g = 0; g < nd; ++g) {
+          const float2 w = f[g * hr * ld];
+          const float c = (up ? w.y : w.x) * inv;
+          v1 += c;
+          v2 = fmaf(c, c, v2);
           if constexpr (EPI == EPI_TOPK) {
-            if (c > bst[q]) {
-              bst[q] = c;
-              barg[q] = angle * a.nt_total + a.n0 + d;
+            if (c > b) {
+              b = c;
+              arg = d0 + g;
             }
           }
         }
-      } else if constexpr (EPI == EPI_CHUNK) {
-        bool hit = false;
-        for (int q = t; q < npix; q += 256) {
-          const int r = q / L, ox = q - r * L, x = ox + L / 2 - (ox + L / 2 >= L ? L : 0);
-          const float2 w = f[(size_t)(r < hr ? r : r - hr) * ld + x];
-          const float z = ((r < hr ? w.x : w.y) * inv - ms[q].x) * ms[q].y;
-          hit = hit || z >= a.thresh;
+        s1[q] = v1;
+        s2[q] = v2;
+        if constexpr (EPI == EPI_TOPK) {
+          if (arg >= 0) {
+            bst[q] = b;
+            barg[q] = angle * a.nt_total + a.n0 + arg;
+          }
         }
-        if (__syncthreads_or(hit)) {  // CTA-uniform
+      }
+    }
+    if constexpr (EPI == EPI_CHUNK) {
+      unsigned hit = 0;
+      for (int q = t; q < npix; q += 256) {
+        bool up;
+        const float2* f = fg + place(q, up);
+        const float2 m = ms[q];
+        for (int g = 0; g < nd; ++g) {
+          const float2 w = f[g * hr * ld];
+          if (((up ? w.y : w.x) * inv - m.x) * m.y >= a.thresh) hit |= 1u << g;
+        }
+      }
+      hit = __reduce_or_sync(0xffffffffu, hit);
+      if (lane == 0 && hit) atomicOr(&hits, hit);
+      __syncthreads();
+    }
+
+    for (int g = 0; g < nd; ++g) {
+      const int d = d0 + g, p = e * a.D + d;
+      const float2* f = fg + g * hr * ld;
+
+      if constexpr (EPI == EPI_CHUNK) {
+        if (hits >> g & 1) {  // CTA-uniform
           for (int i = 0; i < nch; ++i) {
             const int q = 256 * i + t;
-            const int r = q / L, ox = q - r * L, x = ox + L / 2 - (ox + L / 2 >= L ? L : 0);
-            const float2 w = f[(size_t)(r < hr ? r : r - hr) * ld + x];
-            const float z = ((r < hr ? w.x : w.y) * inv - ms[q].x) * ms[q].y;
+            bool up;
+            const float2 w = f[place(q, up)];
+            const float z = ((up ? w.y : w.x) * inv - ms[q].x) * ms[q].y;
             unsigned long long key = ((unsigned long long)float_key(z) << 32) | (unsigned)(255 - brev8(t));
             for (int off = 16; off > 0; off >>= 1) {
               const unsigned long long o = __shfl_xor_sync(0xffffffffu, key, off);
@@ -359,14 +409,16 @@ __global__ void __launch_bounds__(256) gen_rows_kernel(const float2* __restrict_
             cd.pad = 0;
             a.cand[slot] = cd;
           }
+          __syncthreads();  // reduction slots reused next
         }
       } else if constexpr (EPI == EPI_NONORM) {
         double t1 = 0.0, t2 = 0.0;
         for (int i = 0; i < nch; ++i) {
           const int q = 256 * i + t;
-          const int r = q / L, ox = q - r * L, oy = Y0 + r, x = ox + L / 2 - (ox + L / 2 >= L ? L : 0);
-          const float2 w = f[(size_t)(r < hr ? r : r - hr) * ld + x];
-          const float v = r < hr ? w.x : w.y;
+          const int r = fast_div(q, div_l), ox = q - r * L, oy = Y0 + r;
+          bool up;
+          const float2 w = f[place(q, up)];
+          const float v = up ? w.y : w.x;
           t1 += v;
           t2 += (double)v * v;
           float val = v;
@@ -407,15 +459,15 @@ __global__ void __launch_bounds__(256) gen_rows_kernel(const float2* __restrict_
                                          ((unsigned long long)(0xFFFFFu - chunk) << 8) | (best & 0xffu));
           }
         }
+        __syncthreads();  // reduction slots reused next
       } else if constexpr (EPI == EPI_MAP) {
         float* out = a.map_out + (size_t)p * L2 + (size_t)Y0 * L;
         for (int q = t; q < npix; q += 256) {
-          const int r = q / L, ox = q - r * L, x = ox + L / 2 - (ox + L / 2 >= L ? L : 0);
-          const float2 w = f[(size_t)(r < hr ? r : r - hr) * ld + x];
-          out[q] = (r < hr ? w.x : w.y) * inv;
+          bool up;
+          const float2 w = f[place(q, up)];
+          out[q] = (up ? w.y : w.x) * inv;
         }
       }
-      if constexpr (EPI == EPI_CHUNK || EPI == EPI_NONORM) __syncthreads();  // reduction slots reused next
     }
     __syncthreads();  // the transform buffers are rewritten next
   }
@@ -433,8 +485,12 @@ __global__ void __launch_bounds__(256) gen_rows_kernel(const float2* __restrict_
   }
 }
 
+// Row stride in shared memory: the loads write hr rows of a column at a time, 16 / hr columns per
+// half warp, to distinct banks.
+int gen_rows_ld(int L, int RB) { return L + std::max(1, 16 / (RB / 2)); }
+
 size_t gen_rows_smem(int L, int RB, int epi, int tb) {
-  const size_t ld = (size_t)L + 1, npix = (size_t)RB * L, nch = npix / 256;
+  const size_t ld = gen_rows_ld(L, RB), npix = (size_t)RB * L, nch = npix / 256;
   size_t b = sizeof(float2) * tb * RB * ld + sizeof(unsigned long long) * nch * 8 + sizeof(double) * 16;
   if (epi == EPI_SUM || epi == EPI_TOPK) b += 16 * npix;
   if (epi == EPI_CHUNK) b += sizeof(float2) * npix;
@@ -442,29 +498,28 @@ size_t gen_rows_smem(int L, int RB, int epi, int tb) {
 }
 
 constexpr size_t kGenSmemMax = 200 * 1024;
+constexpr int kGenColPoints = 5632;  // per CTA of the column pass (88 KB: two CTAs per SM)
 
-// Templates per transform pass of gen_rows_kernel: up to kGenTB as the shared memory allows.
-constexpr int kGenTB = 4;
-int gen_rows_tb(int L, int RB, int epi) {
-  int tb = kGenTB;
-  while (tb > 1 && gen_rows_smem(L, RB, epi, tb) > kGenSmemMax) tb /= 2;
-  return tb;
+// Templates per transform pass of gen_rows_kernel: as fill its CTA's passes best (smooth_rows), three
+// CTAs per SM where one template's rows leave room for that.
+constexpr int kGenTB = 16;
+int gen_rows_tb(int L, int RB, int epi, const SmoothPlan& plan) {
+  const size_t one = gen_rows_smem(L, RB, epi, 1), two = gen_rows_smem(L, RB, epi, 2);
+  const size_t room = kGenSmemMax / 3 > one ? kGenSmemMax / 3 - one : 0;
+  const int tb = std::min<long long>(kGenTB, 1 + room / (two - one));
+  return smooth_rows(plan, L, 256, tb * (RB / 2) * L, RB / 2) / (RB / 2);
 }
 
-// The row kernels of one epilogue (compiled for L = 320, and for any L): raises their dynamic
-// shared-memory limit to kGenSmemMax once per device, at the first launch that needs more
-// than the default 48 KB (the first angle of a sweep runs before any graph capture), and
-// returns the one for L.
-template <auto K320, auto KANY>
-auto gen_rows_pick(int L, size_t smem) {
+// A row kernel with its dynamic shared-memory limit raised to kGenSmemMax, once per device, at the
+// first launch that needs more than the default 48 KB (the first angle of a sweep runs before any
+// graph capture).
+template <auto K>
+auto gen_kernel(size_t smem) {
   if (smem > 48 * 1024) {
     static PerDeviceOnce once;
-    once([] {
-      GISSPA_CUDA(cudaFuncSetAttribute(K320, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGenSmemMax));
-      GISSPA_CUDA(cudaFuncSetAttribute(KANY, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGenSmemMax));
-    });
+    once([] { GISSPA_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGenSmemMax)); });
   }
-  return L == 320 ? K320 : KANY;
+  return K;
 }
 
 }  // namespace
@@ -472,7 +527,7 @@ auto gen_rows_pick(int L, size_t smem) {
 bool generic_fused(int L, int epi) {
   if (L > kSmoothMax || smooth_plan(L).ns == 0) return false;
   const int rb = gen_rows_rb(L, epi);
-  return rb > 0 && gen_rows_smem(L, rb, epi, 1) <= kGenSmemMax && (size_t)2 * sizeof(float2) * L <= kGenSmemMax;
+  return rb > 0 && gen_rows_smem(L, rb, epi, 1) <= kGenSmemMax && (size_t)2 * sizeof(float2) * (L + kGenColPad) <= kGenSmemMax;
 }
 
 bool correlate_fast(int L) { return L == 256 || L == 320 || L == 512 || L == 1024; }
@@ -488,47 +543,35 @@ void correlate_generic(const CorrLaunch& cl, const float2* I, const void* T, con
   if (generic_fused(L, cl.epi)) {
     const SmoothPlan plan = smooth_plan(L);
     const float2* tw = fft.twiddles(L);
-    const long long nrows = (long long)P * (L / 2 + 1);
-    const int rpc = std::max(1, 2048 / L);
-    const size_t smc = 2 * sizeof(float2) * (size_t)rpc * L;
-    const unsigned gc = (unsigned)((nrows + rpc - 1) / rpc);
-    // L = 320, the reference's default window size, runs kernels compiled for that length
-    // at most 2048 points per CTA: 32 KB, within the default shared-memory limit
-    auto cols = [&](auto k320, auto kany, const auto* t) {
-      auto kernel = L == 320 ? k320 : kany;
-      kernel<<<gc, 256, smc, s>>>(I, t, a.b0, a.n0, cl.D, L, nrows, rpc, plan, tw, z);
+    const unsigned div_l = fast_div_mul(L);
+    const int nrows = P * (L / 2 + 1);
+    const int rpc = std::min(kGenMaxCols, smooth_rows(plan, L, 256, kGenColPoints));
+    const size_t smc = 2 * sizeof(float2) * (size_t)rpc * (L + kGenColPad);
+    const unsigned gc = (unsigned)ceil_div(nrows, rpc);
+    auto cols = [&](auto kernel, const auto* t) {
+      kernel<<<gc, 256, smc, s>>>(I, t, a.b0, a.n0, cl.D, L, div_l, nrows, rpc, plan, tw, z);
     };
     switch (cl.spec) {
-      case GISSPA_SPEC_FP32:
-        cols(gen_cols_kernel<320, SpecFp32>, gen_cols_kernel<0, SpecFp32>, static_cast<const float2*>(T));
-        break;
-      case GISSPA_SPEC_FP16:
-        cols(gen_cols_kernel<320, SpecFp16>, gen_cols_kernel<0, SpecFp16>, static_cast<const __half2*>(T));
-        break;
+      case GISSPA_SPEC_FP32: cols(gen_kernel<gen_cols_kernel<SpecFp32>>(smc), static_cast<const float2*>(T)); break;
+      case GISSPA_SPEC_FP16: cols(gen_kernel<gen_cols_kernel<SpecFp16>>(smc), static_cast<const __half2*>(T)); break;
       case GISSPA_SPEC_BF16:
-        cols(gen_cols_kernel<320, SpecBf16>, gen_cols_kernel<0, SpecBf16>, static_cast<const __nv_bfloat162*>(T));
+        cols(gen_kernel<gen_cols_kernel<SpecBf16>>(smc), static_cast<const __nv_bfloat162*>(T));
         break;
       default: throw CudaError{cudaErrorInvalidValue, "unknown spectrum precision"};
     }
     GISSPA_LAUNCH_CHECK();
     if (ev) GISSPA_CUDA(cudaEventRecord(ev[1], s));
-    const int rb = gen_rows_rb(L, cl.epi);
-    const int tb = gen_rows_tb(L, rb, cl.epi);
+    const int rb = gen_rows_rb(L, cl.epi), ld = gen_rows_ld(L, rb);
+    const int tb = std::min(gen_rows_tb(L, rb, cl.epi, plan), cl.D);
     const size_t smr = gen_rows_smem(L, rb, cl.epi, tb);
     const dim3 gr((unsigned)(L / rb), (unsigned)cl.E);
-    auto rows = [&](auto kernel) { kernel<<<gr, 256, smr, s>>>(z, a, L, rb, tb, plan, tw); };
+    auto rows = [&](auto kernel) { kernel<<<gr, 256, smr, s>>>(z, a, L, div_l, rb, ld, tb, plan, tw); };
     switch (cl.epi) {
-      case EPI_SUM: rows(gen_rows_pick<gen_rows_kernel<320, EPI_SUM>, gen_rows_kernel<0, EPI_SUM>>(L, smr)); break;
-      case EPI_TOPK:
-        rows(gen_rows_pick<gen_rows_kernel<320, EPI_TOPK>, gen_rows_kernel<0, EPI_TOPK>>(L, smr));
-        break;
-      case EPI_CHUNK:
-        rows(gen_rows_pick<gen_rows_kernel<320, EPI_CHUNK>, gen_rows_kernel<0, EPI_CHUNK>>(L, smr));
-        break;
-      case EPI_NONORM:
-        rows(gen_rows_pick<gen_rows_kernel<320, EPI_NONORM>, gen_rows_kernel<0, EPI_NONORM>>(L, smr));
-        break;
-      case EPI_MAP: rows(gen_rows_pick<gen_rows_kernel<320, EPI_MAP>, gen_rows_kernel<0, EPI_MAP>>(L, smr)); break;
+      case EPI_SUM: rows(gen_kernel<gen_rows_kernel<EPI_SUM>>(smr)); break;
+      case EPI_TOPK: rows(gen_kernel<gen_rows_kernel<EPI_TOPK>>(smr)); break;
+      case EPI_CHUNK: rows(gen_kernel<gen_rows_kernel<EPI_CHUNK>>(smr)); break;
+      case EPI_NONORM: rows(gen_kernel<gen_rows_kernel<EPI_NONORM>>(smr)); break;
+      case EPI_MAP: rows(gen_kernel<gen_rows_kernel<EPI_MAP>>(smr)); break;
       default: throw CudaError{cudaErrorInvalidValue, "unknown epilogue"};
     }
     GISSPA_LAUNCH_CHECK();

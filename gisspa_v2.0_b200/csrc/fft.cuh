@@ -163,6 +163,84 @@ struct Dft<10, SIGN> : DftAB<2, 5, SIGN> {};
 template <int SIGN>
 struct Dft<20, SIGN> : DftAB<4, 5, SIGN> {};
 
+
+// 3-point DFT: X_1, X_2 = x0 - t / 2 +- SIGN i sin(2 pi / 3) u with t = x1 + x2, u = x1 - x2
+template <int SIGN>
+struct Dft<3, SIGN> {
+  __device__ __forceinline__ static void run(float2* a) {
+    constexpr float s = 0.86602540378443864676f;
+    const float2 t = cadd(a[1], a[2]), u = csub(a[1], a[2]);
+    const float2 p = pfma(t, make_float2(-0.5f, -0.5f), a[0]);
+    const float2 iq = pmul(make_float2(-SIGN * s, SIGN * s), make_float2(u.y, u.x));
+    a[0] = cadd(a[0], t);
+    a[1] = cadd(p, iq);
+    a[2] = csub(p, iq);
+  }
+};
+
+// 7-point DFT from the symmetric pairs t_j = x_j + x_{7-j}, u_j = x_j - x_{7-j}, as Dft<5>
+template <int SIGN>
+struct Dft<7, SIGN> {
+  __device__ __forceinline__ static void run(float2* a) {
+    // cos and sin of 2 pi j / 7, j = 1..3
+    constexpr float c[3] = {0.62348980185873353053f, -0.22252093395631440429f, -0.90096886790241912624f};
+    constexpr float s[3] = {0.78183148246802980871f, 0.97492791218182360702f, 0.43388373911755812048f};
+    float2 t[3], u[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      t[j] = cadd(a[j + 1], a[6 - j]);
+      const float2 d = csub(a[j + 1], a[6 - j]);
+      u[j] = make_float2(-SIGN * d.y, SIGN * d.x);  // SIGN i u_j
+    }
+    const float2 x0 = a[0];
+    a[0] = cadd(cadd(x0, t[0]), cadd(t[1], t[2]));
+#pragma unroll
+    for (int k = 1; k <= 3; ++k) {
+      float2 p = x0, q = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int j = 1; j <= 3; ++j) {
+        const int m = j * k % 7, f = m > 3 ? 7 - m : m;  // cos is even, sin odd
+        const float cc = c[f - 1], ss = m > 3 ? -s[f - 1] : s[f - 1];
+        p = pfma(t[j - 1], make_float2(cc, cc), p);
+        q = j == 1 ? pmul(u[0], make_float2(ss, ss)) : pfma(u[j - 1], make_float2(ss, ss), q);
+      }
+      a[k] = cadd(p, q);
+      a[7 - k] = csub(p, q);
+    }
+  }
+};
+
+// Length A B with A, B coprime, without inner twiddles (Good and Thomas): x[(B n1 + A n2) mod AB]
+// through B-point and A-point transforms gives X[k] at k mod A, k mod B.
+template <int A, int B, int SIGN>
+struct DftPfa {
+  __device__ __forceinline__ static void run(float2* a) {
+    float2 y[A][B], z[B][A];
+#pragma unroll
+    for (int n1 = 0; n1 < A; ++n1) {
+#pragma unroll
+      for (int n2 = 0; n2 < B; ++n2) y[n1][n2] = a[(B * n1 + A * n2) % (A * B)];
+      Dft<B, SIGN>::run(y[n1]);
+    }
+#pragma unroll
+    for (int k2 = 0; k2 < B; ++k2) {
+#pragma unroll
+      for (int n1 = 0; n1 < A; ++n1) z[k2][n1] = y[n1][k2];
+      Dft<A, SIGN>::run(z[k2]);
+    }
+#pragma unroll
+    for (int k = 0; k < A * B; ++k) a[k] = z[k % B][k % A];
+  }
+};
+template <int SIGN>
+struct Dft<6, SIGN> : DftPfa<2, 3, SIGN> {};
+template <int SIGN>
+struct Dft<12, SIGN> : DftPfa<4, 3, SIGN> {};
+template <int SIGN>
+struct Dft<14, SIGN> : DftPfa<2, 7, SIGN> {};
+template <int SIGN>
+struct Dft<15, SIGN> : DftPfa<3, 5, SIGN> {};
+
 // In-register DFT of length R (R in {1, 2, 4, 8, 16}), natural order in and out.
 template <int R, int SIGN>
 struct Dft {

@@ -1,4 +1,5 @@
 // fft_generic.cu — batched FFTs outside the hot loop (see fft_generic.cuh).
+#include <algorithm>
 #include <cmath>
 #include <complex>
 
@@ -189,6 +190,66 @@ void host_fft_pow2(std::vector<std::complex<double>>& x, int sign) {
 
 }  // namespace
 
+namespace {
+// Radices r[0..ns) <= top with product n, ns given: the first found has the smallest largest radix
+// when the caller raises `top` step by step.
+bool smooth_split(int n, int ns, int top, int* r) {
+  if (ns == 0) return n == 1;
+  for (int i = top; i >= 0; --i) {
+    const int R = kSmoothRadices[i];
+    if (n % R == 0 && smooth_split(n / R, ns - 1, i, r + 1)) {
+      r[0] = R;
+      return true;
+    }
+  }
+  return false;
+}
+}  // namespace
+
+SmoothPlan smooth_plan(int n) {
+  SmoothPlan p;
+  int rest = n;
+  for (int f : {2, 3, 5, 7})
+    while (rest > 1 && rest % f == 0) rest /= f;
+  if (n < 2 || rest != 1) return p;
+  constexpr int kR = sizeof(kSmoothRadices) / sizeof(int);
+  for (int ns = 1; ns <= SmoothPlan::kMax && !p.ns; ++ns)
+    for (int top = 0; top < kR; ++top)
+      if (smooth_split(n, ns, top, p.r)) {
+        p.ns = ns;
+        break;
+      }
+  std::sort(p.r, p.r + p.ns, [](int a, int b) {
+    const int va = a & -a, vb = b & -b;  // powers of two in the radices
+    return va != vb ? va < vb : a < b;
+  });
+  int Ns = 1;
+  for (int s = 0; s < p.ns; ++s) {
+    p.div_m[s] = fast_div_mul(n / p.r[s]);
+    p.div_ns[s] = fast_div_mul(Ns);
+    Ns *= p.r[s];
+  }
+  return p;
+}
+
+int smooth_rows(const SmoothPlan& plan, int n, int threads, int max_points, int step) {
+  int best = step;
+  double fill = 0;
+  for (int rows = step; rows == step || (long long)rows * n <= max_points; rows += step) {
+    double used = 0, held = 0;
+    for (int s = 0; s < plan.ns; ++s) {  // a pass costs about its radix
+      const double nb = (double)rows * (n / plan.r[s]), passes = std::ceil(nb / threads);
+      used += nb * plan.r[s];
+      held += passes * threads * plan.r[s];
+    }
+    if (used / held > fill + 0.01) {
+      fill = used / held;
+      best = rows;
+    }
+  }
+  return best;
+}
+
 const float2* FftEngine::twiddles(int n) {
   auto it = tw_.find(n);
   if (it != tw_.end()) return it->second.as<float2>();
@@ -282,7 +343,7 @@ void FftEngine::rows(float2* data, long long nrows, int n, int sign, float scale
   }
   const SmoothPlan sp = n <= kSmoothMax ? smooth_plan(n) : SmoothPlan{};
   if (sp.ns > 0) {
-    const int rpc = n >= 2048 ? 1 : 2048 / n;
+    const int rpc = smooth_rows(sp, n, 256, 4096);
     const size_t smem = 2 * sizeof(float2) * (size_t)rpc * n;
     const float2* tw = twiddles(n);
     const long long grid = (nrows + rpc - 1) / rpc;

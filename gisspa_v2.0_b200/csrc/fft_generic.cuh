@@ -64,31 +64,26 @@ class DevBuf {
   size_t n_ = 0;
 };
 
-// Radices (4 first, then 2, 3, 5, 7) whose product is n; ns = 0 when n has a prime factor
-// above 7 (such lengths use Bluestein's algorithm).
+// Stockham stages of a row of length n: radices from kSmoothRadices (register transforms of that
+// length) whose product is n, as few as possible, the largest as small as possible; ns = 0 when n
+// has a prime factor above 7 (such lengths use Bluestein's algorithm).  Odd radices come first: the
+// first stage writes its outputs R apart, in distinct banks for odd R.
+constexpr int kSmoothRadices[] = {2, 3, 4, 5, 6, 7, 8, 10, 12, 14, 15, 16};
 struct SmoothPlan {
-  static constexpr int kMax = 16;
+  static constexpr int kMax = 13;  // radices of 2^13
   int ns = 0;
   int r[kMax] = {};
+  unsigned div_m[kMax] = {}, div_ns[kMax] = {};  // fast_div of n / r and of the radices before
 };
-__host__ __device__ constexpr SmoothPlan smooth_plan_c(int n) {
-  SmoothPlan p;
-  if (n < 2) return p;
-  const int fs[5] = {4, 2, 3, 5, 7};
-  int rest = n;
-  while (rest % 4 == 0 && rest > 4 && p.ns < SmoothPlan::kMax) {
-    p.r[p.ns++] = 4;
-    rest /= 4;
-  }
-  for (int i = 0; i < 5; ++i)
-    while (rest % fs[i] == 0 && p.ns < SmoothPlan::kMax) {
-      p.r[p.ns++] = fs[i];
-      rest /= fs[i];
-    }
-  if (rest != 1) p.ns = 0;
-  return p;
+// i / d for i d < 2^32 (mul: fast_div_mul(d))
+__host__ __device__ constexpr unsigned fast_div_mul(unsigned d) {
+  return d > 1 ? (unsigned)(((1ull << 32) + d - 1) / d) : 0;
 }
-inline SmoothPlan smooth_plan(int n) { return smooth_plan_c(n); }
+__device__ __forceinline__ int fast_div(int i, unsigned mul) { return mul ? (int)__umulhi((unsigned)i, mul) : i; }
+SmoothPlan smooth_plan(int n);
+// Rows of length n per CTA of `threads`, a multiple of `step`, of at most max_points points (or
+// `step`): the count whose butterflies fill the CTA's passes best.
+int smooth_rows(const SmoothPlan& plan, int n, int threads, int max_points, int step = 1);
 // Longest row the mixed-radix kernel takes (two shared-memory copies of 8192 complex = 128 KB).
 constexpr int kSmoothMax = 8192;
 
