@@ -1757,10 +1757,10 @@ void refine_run(gisspa_handle* h, gisspa_pick* picks, size_t n, int steps, gissp
   if (ctf) *ctf = ctf_of(psi);
 }
 
-// All windows and a few templates per launch, as many pairs as keep their intermediate in L2
-// beside the spectra: with every template of one window per launch, 24 pairs of window 1024 wrote
-// and read 100 MB of it through DRAM.
-constexpr size_t kMapBatchBytes = 32u << 20;
+// All windows and a few templates per launch: a template's spectrum is read once for all windows,
+// and the launches are large beside their last waves.  96 pairs of window 1024: 389 us with 32 MB
+// of intermediate per launch, 386 with 64, 349 with 128, 347 with 256.
+constexpr size_t kMapBatchBytes = 128u << 20;
 void cc_maps(gisspa_handle* h, const void* d_win, int nw, const void* d_t, int ntm, int spec, float* d_out) {
   Ctx c{h, h->stream, h->cfg.window_size, (long long)h->cfg.window_size * h->cfg.window_size, DevParams{}};
   const int l = c.l;
