@@ -66,6 +66,13 @@ struct ColXform<320, 16> {
   }
 };
 
+template <int TEAM>
+__device__ __forceinline__ double team_sum_f64(double x) {
+#pragma unroll
+  for (int off = TEAM / 2; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off, TEAM);
+  return x;
+}
+
 // Pass A: one team of TT threads per column slot, NC slots per CTA, one pair per blockIdx.y.
 // Each column is a two-stage Stockham transform (32 x 16 points at L = 512) with E = L / TT
 // points per thread: one exchange through the team's slice of shared memory, inside a warp.
@@ -75,11 +82,18 @@ struct ColXform<320, 16> {
 // of NC slots leaves as contiguous 16-byte stores.  The swizzle key is y >> SH with 16 / NC =
 // 2^SH rows per 128-byte line, so 16 consecutive rows of one column fall in 16 distinct bank
 // pairs.
-template <int L, typename SPEC, int V = 0>
+// NN: adds each pair's sums over its map to nn, from the products Z themselves: the raw map's sum
+// is L^2 Z(0), its sum of squares L^2 sum |Z|^2 over the whole plane (columns 0 < kx < L/2 of the
+// half plane count twice).
+struct MapSums {
+  double* sum;   // [window][nt_total][2]
+  int nt_total;
+};
+template <int L, typename SPEC, int V = 0, bool NN = false>
 __device__ __forceinline__ void pass_a_body(float2* smem, const float2* __restrict__ I,
                                             const typename SPEC::T* __restrict__ T, float2* __restrict__ Q, int b0,
                                             int n0, int D, const float2* __restrict__ twL, int p, int cgroup,
-                                            bool wait_before_store, const SkipMask& sk) {
+                                            bool wait_before_store, const SkipMask& sk, const MapSums& nn = MapSums{}) {
   constexpr int TT = PassA<L, V>::TT, NC = PassA<L, V>::NC, E = L / TT, NZ = L / 2, HS = NZ + 1;
   using CX = ColXform<L, TT>;
   constexpr int SH = NC >= 16 ? 0 : NC == 8 ? 1 : 2;
@@ -95,6 +109,8 @@ __device__ __forceinline__ void pass_a_body(float2* smem, const float2* __restri
   const float2* Ib = I + (size_t)(b0 + e) * HS * L;
   const typename SPEC::T* Tn = T + (size_t)(n0 + d) * HS * L;
   float2 v[E];
+  double sq = 0.0;
+  double* sums = NN ? nn.sum + 2 * ((size_t)(b0 + e) * nn.nt_total + n0 + d) : nullptr;
   if (c == 0) {
     // columns kx = 0 and kx = L/2 have real inverse transforms: pack them as a + i b
 #pragma unroll
@@ -103,6 +119,10 @@ __device__ __forceinline__ void pass_a_body(float2* smem, const float2* __restri
       const float2 a = cmulc(Ib[ky], SPEC::load(Tn + ky));
       const float2 b = cmulc(Ib[(size_t)NZ * L + ky], SPEC::load(Tn + (size_t)NZ * L + ky));
       v[i] = make_float2(a.x - b.y, a.y + b.x);
+      if constexpr (NN) {
+        sq += (double)a.x * a.x + (double)a.y * a.y + (double)b.x * b.x + (double)b.y * b.y;
+        if (ky == 0) atomicAdd(sums, (double)a.x * ((double)L * L));
+      }
     }
   } else {
     const float2* Ic = Ib + (size_t)c * L;
@@ -111,10 +131,23 @@ __device__ __forceinline__ void pass_a_body(float2* smem, const float2* __restri
     for (int i = 0; i < E; ++i) {
       const int ky = CX::in_index(tid, i);
       v[i] = cmulc(__ldg(Ic + ky), SPEC::load(Tc + ky));
+      if constexpr (NN) sq += 2.0 * ((double)v[i].x * v[i].x + (double)v[i].y * v[i].y);
     }
+  }
+  __shared__ double nn_part[NN ? NC : 1];
+  if constexpr (NN) {
+    sq = team_sum_f64<TT>(sq);
+    if (tid == 0) nn_part[team] = sq;
   }
   CX::run(v, smem + team * L, twL, tid);
   __syncthreads();
+  if constexpr (NN) {
+    if (threadIdx.x == 0) {
+      sq = 0.0;
+      for (int q = 0; q < NC; ++q) sq += nn_part[q];
+      atomicAdd(sums + 1, sq * ((double)L * L));
+    }
+  }
 #pragma unroll
   for (int i = 0; i < E; ++i) {
     const int y = CX::out_index(tid, i);
@@ -150,12 +183,6 @@ template <int W>
 __device__ __forceinline__ float group_max(float x) {
 #pragma unroll
   for (int off = W / 2; off > 0; off >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, off, W));
-  return x;
-}
-template <int TEAM>
-__device__ __forceinline__ double team_sum_f64(double x) {
-#pragma unroll
-  for (int off = TEAM / 2; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off, TEAM);
   return x;
 }
 template <int TEAM>

@@ -9,14 +9,15 @@ namespace gisspa {
 namespace {
 
 // Pass A kernel: one pair per blockIdx.y, NC column slots per blockIdx.x (pass_a_body).
-template <int L, typename SPEC, int V>
+// NN: EPI_NONORM's sums too.
+template <int L, typename SPEC, int V, bool NN>
 __global__ void __launch_bounds__(PassA<L, V>::TT * PassA<L, V>::NC, PassA<L, V>::MINB)
     pass_a_kernel(const float2* __restrict__ I, const typename SPEC::T* __restrict__ T, float2* __restrict__ Q,
-                  int b0, int n0, int D, const float2* __restrict__ twL, int chained, SkipMask sk) {
+                  int b0, int n0, int D, const float2* __restrict__ twL, int chained, SkipMask sk, MapSums nn) {
   extern __shared__ __align__(16) float2 smem[];  // [NC * L]: FFT exchange buffers, then the output tile
   griddep_launch_dependents();
   if (!chained) griddep_wait();  // the spectra may come from the kernel just before
-  pass_a_body<L, SPEC, V>(smem, I, T, Q, b0, n0, D, twL, blockIdx.y, blockIdx.x, chained != 0, sk);
+  pass_a_body<L, SPEC, V, NN>(smem, I, T, Q, b0, n0, D, twL, blockIdx.y, blockIdx.x, chained != 0, sk, nn);
 }
 
 // Pass A of a pruned second sweep: one CTA per pair looping over the column groups, so that the
@@ -202,7 +203,6 @@ __global__ void __launch_bounds__(NW * 32, MINB)
       return;
     }
     float2* stg = stage + (k & 1) * RB * NZ;
-    double nn_s1 = 0.0, nn_s2 = 0.0;
 #pragma unroll
     for (int s = 0; s < RPT; ++s) {
       const int r = team + NTEAM * s;
@@ -324,46 +324,6 @@ __global__ void __launch_bounds__(NW * 32, MINB)
               for (int ch = 0; ch < CPR; ++ch) emit_chunk<L>(a, keys[ch], c0 + ch, win, a.n0 + d, angle);
           }
         }
-      } else if constexpr (EPI == EPI_NONORM) {
-        static_assert(TEAM <= 32, "peak and sums reduce within a warp");
-        constexpr int CPR = L % 256 == 0 ? L / 256 : 2;
-        const int c0 = (oy * L) >> 8;
-        // get_peak_and_SUM (kernels.cu:725-763): sums over every pixel, max with the
-        // border (closer than diameter/4 to the window edge) forced to 0
-#pragma unroll
-        for (int i = 0; i < E; ++i) {
-          nn_s1 += (double)v[i].x + (double)v[i].y;
-          nn_s2 += (double)v[i].x * v[i].x + (double)v[i].y * v[i].y;
-        }
-#pragma unroll
-        for (int ch = 0; ch < CPR; ++ch) {
-          unsigned long long key = 0;
-#pragma unroll
-          for (int i = 0; i < E; ++i)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int x = ox[i] + h;
-              if (((oy * L + x) >> 8) - c0 != ch) continue;
-              float val = h ? v[i].y : v[i].x;
-              if (x < a.border || x > L - a.border || oy < a.border || oy > L - a.border) val = 0.f;
-              const int t = (oy * L + x) & 255;
-              const unsigned long long k2 =
-                  ((unsigned long long)float_key(val) << 32) | (unsigned)(255 - brev8(t));
-              key = k2 > key ? k2 : key;
-            }
-          key = team_max_u64<TEAM>(key);
-          if (lt == 0) {
-            const float vb = key_float((uint32_t)(key >> 32));
-            if (vb > 0.f) {
-              // largest value, then the lowest chunk, then the reference's in-chunk order (the
-              // byte 255 - brev8(t)): parts of one chunk from two rows combine correctly
-              const int chunk = c0 + ch;
-              const unsigned long long g = ((unsigned long long)float_key(vb) << 32) |
-                                           ((unsigned long long)(0xFFFFFu - chunk) << 8) | (key & 0xffu);
-              atomicMax(a.nn_key + (size_t)win * a.nt_total + a.n0 + d, g);
-            }
-          }
-        }
       }
     }
     if constexpr (EPI == EPI_CHUNK && L % 256 != 0) {
@@ -372,15 +332,6 @@ __global__ void __launch_bounds__(NW * 32, MINB)
         const unsigned long long key = chunk_part[q];
         chunk_part[q] = 0ull;
         if (key) emit_chunk<L>(a, key, cbase + q, win, a.n0 + d, angle);
-      }
-    }
-    if constexpr (EPI == EPI_NONORM) {
-      nn_s1 = team_sum_f64<TEAM>(nn_s1);
-      nn_s2 = team_sum_f64<TEAM>(nn_s2);
-      if (lt == 0) {
-        const size_t q = (size_t)win * a.nt_total + a.n0 + d;
-        atomicAdd(a.nn_sum + 2 * q, nn_s1);
-        atomicAdd(a.nn_sum + 2 * q + 1, nn_s2);
       }
     }
     __syncthreads();  // this stage buffer is refilled two templates later
@@ -439,7 +390,12 @@ void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaSt
   ++launch_counter();
 }
 
-constexpr int kMapGroups = 148 * 16;  // CTAs of one row per team below which a launch keeps them
+// Rows per team where a launch then still has `ctas` CTAs, groups rows of teams per pair.
+int rows_per_team(int pairs, int groups, int most, int ctas) {
+  while (most > 1 && (groups % most || (long long)pairs * groups / most < ctas)) most /= 2;
+  return most;
+}
+
 // Pass B of EPI_MAP: the pairs of a launch are independent (nothing is summed over templates), so
 // every row of every pair is a team's own work: teams load their rows themselves, without the bulk
 // copies and their bounded waits.  `per` rows per team share the CTA's tables.
@@ -490,9 +446,115 @@ __global__ void __launch_bounds__(MapShape<L>::NW * 32)
 template <int L>
 void launch_map(const CorrLaunch& cl, const CorrArgs& args, const float2* twL, const float2* twNZ, cudaStream_t s) {
   constexpr int G = L / MapShape<L>::NTEAM;  // row groups per pair
-  const int per = (long long)cl.D * cl.E * G >= kMapGroups ? 4 : 1;
-  static_assert(G % 4 == 0, "whole CTAs per pair");
+  const int per = rows_per_team(cl.D * cl.E, G, 4, 148 * 4);
   launch_pdl(map_rows_kernel<L>, dim3(G / per, cl.D * cl.E), dim3(MapShape<L>::NW * 32), 0, s, args, per, twL, twNZ);
+}
+
+// Pass B of EPI_NONORM (get_peak_and_SUM, kernels.cu:725-763): each pair's peak, with the border
+// (closer than diameter/4 to the window edge) forced to 0.  A team takes `per` rows of one pair, as
+// in the map kernel; the sums come from pass A's spectra (MapSums).  The scan for the peak's place
+// in the reference's order of 256-pixel chunks runs only for rows whose largest value is at least
+// the CTA's and, as far as it has been seen, the pair's.  With the sums of every pixel in FP64, the
+// scan of every row and the templates in step behind bulk copies, 96 pairs of window 512 took
+// 52 us; now 43 (pass A, with the sums from its spectra, 49 instead of 44).
+template <int L>
+__global__ void __launch_bounds__(MapShape<L>::NW * 32)
+    nonorm_rows_kernel(CorrArgs a, int per, const float2* __restrict__ twL, const float2* __restrict__ twNZ) {
+  using S = MapShape<L>;
+  using RX = RowXform<L, S::TEAM>;
+  constexpr int NZ = L / 2, TEAM = S::TEAM, NV = NZ / 2 / TEAM, E = RX::EOUT;
+  constexpr int CPR = L % 256 == 0 ? L / 256 : 2;  // chunks that a row touches
+  static_assert(2 * E <= 32, "a bit per pixel");
+  __shared__ __align__(16) float2 rows[S::NTEAM][NZ];
+  __shared__ __align__(16) float2 tw_nz[NZ + NZ / 16], tw_l[NZ];
+  __shared__ unsigned cta_best;  // float_key of the CTA's largest value
+  griddep_launch_dependents();
+  for (int i = threadIdx.x; i < NZ; i += S::NW * 32) {
+    tw_nz[tw_pad_index(i)] = __ldg(twNZ + i);
+    tw_l[i] = __ldg(twL + i);
+  }
+  if (threadIdx.x == 0) cta_best = 0u;
+  __syncthreads();
+  const int team = threadIdx.x / TEAM, lt = threadIdx.x - team * TEAM;
+  const int p = blockIdx.y, e = p / a.D, d = p - e * a.D;
+  float2* row = rows[team];
+  int ox[E];
+  unsigned in_x = 0;  // pixels inside the border, by column
+#pragma unroll
+  for (int i = 0; i < E; ++i) {
+    ox[i] = (2 * RX::out_index(lt, i) + L / 2) % L;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int x = ox[i] + h;
+      in_x |= (x < a.border || x > L - a.border ? 0u : 1u) << (2 * i + h);
+    }
+  }
+  griddep_wait();  // Q comes from the pass A just before
+  unsigned long long* key_out = a.nn_key + (size_t)(a.b0 + e) * a.nt_total + a.n0 + d;
+  const unsigned seen = (unsigned)(__ldcg(key_out) >> 32);
+  const int y0 = blockIdx.x * per * S::NTEAM + team;
+  const float4* src = reinterpret_cast<const float4*>(a.Q + ((size_t)p * L + y0) * NZ) + lt;
+  float4 in[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) in[i] = src[i * TEAM];
+  for (int q = 0; q < per; ++q) {
+    const int oy = (y0 + q * S::NTEAM + L / 2) % L;
+    __syncwarp();  // the row before has been read
+#pragma unroll
+    for (int i = 0; i < NV; ++i) reinterpret_cast<float4*>(row)[lt + i * TEAM] = in[i];
+    __syncwarp();
+    if (q + 1 < per) {
+      src += S::NTEAM * NZ / 2;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) in[i] = src[i * TEAM];
+    }
+    float2 v[RX::EBUF];
+    RX::run(v, row, tw_nz, tw_l, lt, WarpSync{});
+    float vmax = -INFINITY;
+    if (!(oy < a.border || oy > L - a.border)) {
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        vmax = fmaxf(vmax, in_x >> (2 * i) & 1 ? v[i].x : -INFINITY);
+        vmax = fmaxf(vmax, in_x >> (2 * i + 1) & 1 ? v[i].y : -INFINITY);
+      }
+    }
+    const unsigned kmax = __reduce_max_sync(0xffffffffu, float_key(vmax));  // (a warp's rows: one pair's)
+    unsigned best = seen;
+    if ((threadIdx.x & 31) == 0) best = max(best, atomicMax(&cta_best, kmax));
+    best = __shfl_sync(0xffffffffu, best, 0);
+    if (kmax <= float_key(0.f) || kmax < best) continue;
+    const int c0 = (oy * L) >> 8;
+#pragma unroll
+    for (int ch = 0; ch < CPR; ++ch) {
+      unsigned long long key = 0;
+#pragma unroll
+      for (int i = 0; i < E; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int x = ox[i] + h;
+          if (((oy * L + x) >> 8) - c0 != ch) continue;
+          float val = h ? v[i].y : v[i].x;
+          if (!(in_x >> (2 * i + h) & 1) || oy < a.border || oy > L - a.border) val = 0.f;
+          const int t = (oy * L + x) & 255;
+          const unsigned long long k2 = ((unsigned long long)float_key(val) << 32) | (unsigned)(255 - brev8(t));
+          key = k2 > key ? k2 : key;
+        }
+      key = team_max_u64<TEAM>(key);
+      if (lt == 0 && key_float((uint32_t)(key >> 32)) > 0.f) {
+        // largest value, then the lowest chunk, then the reference's in-chunk order (the
+        // byte 255 - brev8(t)): parts of one chunk from two rows combine correctly
+        atomicMax(key_out, (key >> 32 << 32) | ((unsigned long long)(0xFFFFFu - (c0 + ch)) << 8) | (key & 0xffu));
+      }
+    }
+  }
+}
+template <int L>
+void launch_nonorm(const CorrLaunch& cl, const CorrArgs& args, const float2* twL, const float2* twNZ,
+                   cudaStream_t s) {
+  constexpr int G = L / MapShape<L>::NTEAM;
+  const int per = rows_per_team(cl.D * cl.E, G, 8, 148 * 4);
+  launch_pdl(nonorm_rows_kernel<L>, dim3(G / per, cl.D * cl.E), dim3(MapShape<L>::NW * 32), 0, s, args, per, twL,
+             twNZ);
 }
 
 // Pass A's mask: pairs only where pass B lists the live templates (D small enough).
@@ -508,11 +570,12 @@ void launch_a_cfg(const CorrLaunch& cl, const float2* I, const void* T, float2* 
   constexpr int NZ = L / 2;
   using P = PassA<L, V>;
   constexpr size_t smem = (size_t)P::NC * L * sizeof(float2);
-  static PerDeviceOnce once;
-  once([] {
-    GISSPA_CUDA(
-        cudaFuncSetAttribute(pass_a_kernel<L, SPEC, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  });
+  auto launch = [&](auto* kernel, PerDeviceOnce& once, const SkipMask& sk) {
+    once([&] { GISSPA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); });
+    launch_pdl(kernel, dim3(NZ / P::NC, cl.E * cl.D), dim3(P::TT * P::NC), smem, s, I,
+               static_cast<const typename SPEC::T*>(T), Q, args.b0, args.n0, cl.D, twL, cl.chained ? 1 : 0, sk,
+               MapSums{args.nn_sum, args.nt_total});
+  };
   const SkipMask sk = cl.epi == EPI_CHUNK ? a_mask(cl, args) : SkipMask{};
   if (sk.pairs) {
     static PerDeviceOnce once_pair;
@@ -524,9 +587,11 @@ void launch_a_cfg(const CorrLaunch& cl, const float2* I, const void* T, float2* 
                static_cast<const typename SPEC::T*>(T), Q, args.b0, args.n0, cl.D, twL, cl.chained ? 1 : 0, sk);
     return;
   }
-  dim3 grid(NZ / P::NC, cl.E * cl.D);
-  launch_pdl(pass_a_kernel<L, SPEC, V>, grid, dim3(P::TT * P::NC), smem, s, I,
-             static_cast<const typename SPEC::T*>(T), Q, args.b0, args.n0, cl.D, twL, cl.chained ? 1 : 0, sk);
+  static PerDeviceOnce once, once_nn;
+  if (cl.epi == EPI_NONORM)
+    launch(pass_a_kernel<L, SPEC, V, true>, once_nn, sk);
+  else
+    launch(pass_a_kernel<L, SPEC, V, false>, once, sk);
 }
 template <int L, typename SPEC>
 void launch_a(const CorrLaunch& cl, const float2* I, const void* T, float2* Q, const CorrArgs& args,
@@ -597,7 +662,6 @@ void launch_b(const CorrLaunch& cl, const CorrArgs& args, const float2* twL, con
     case EPI_SUMMAX: launch_b_cfg<L, P::TEAM, P::RB, P::NW, EPI_SUMMAX, P::MINB>(cl, args, twL, twNZ, s); break;
     case EPI_CHUNK: launch_b_cfg<L, P::TEAM, P::RB, P::NW, EPI_CHUNK, P::MINB>(cl, args, twL, twNZ, s); break;
     case EPI_TOPK: launch_b_cfg<L, P::TEAM, P::RB, P::NW, EPI_TOPK, P::MINB>(cl, args, twL, twNZ, s); break;
-    case EPI_NONORM: launch_b_cfg<L, P::TEAM, P::RB, P::NW, EPI_NONORM, P::MINB>(cl, args, twL, twNZ, s); break;
     default: throw CudaError{cudaErrorInvalidValue, "unknown epilogue"};
   }
   }
@@ -610,7 +674,7 @@ int launch_pair(const CorrLaunch& cl, const float2* I, const void* T, float2* Q,
   switch (cl.spec) {
     case GISSPA_SPEC_FP32: launch_a<L, SpecFp32>(cl, I, T, Q, args, twL, s); break;
     case GISSPA_SPEC_FP16:
-      if (L == 512 && cl.tc)
+      if (L == 512 && cl.tc && cl.epi != EPI_NONORM)
         launch_a_tc(cl, I, T, Q, args, twL, s);
       else
         launch_a<L, SpecFp16>(cl, I, T, Q, args, twL, s);
@@ -619,8 +683,11 @@ int launch_pair(const CorrLaunch& cl, const float2* I, const void* T, float2* Q,
     default: throw CudaError{cudaErrorInvalidValue, "unknown spectrum precision"};
   }
   if (ev) GISSPA_CUDA(cudaEventRecord(ev[1], s));
-  if (cl.epi == EPI_MAP) {
-    launch_map<L>(cl, args, twL, twNZ, s);
+  if (cl.epi == EPI_MAP || cl.epi == EPI_NONORM) {
+    if (cl.epi == EPI_MAP)
+      launch_map<L>(cl, args, twL, twNZ, s);
+    else
+      launch_nonorm<L>(cl, args, twL, twNZ, s);
     if (ev) GISSPA_CUDA(cudaEventRecord(ev[2], s));
     return 2;
   }

@@ -343,7 +343,8 @@ void FftEngine::rows(float2* data, long long nrows, int n, int sign, float scale
   }
   const SmoothPlan sp = n <= kSmoothMax ? smooth_plan(n) : SmoothPlan{};
   if (sp.ns > 0) {
-    const int rpc = smooth_rows(sp, n, 256, 4096);
+    // (a single image's rows still spread over the chip)
+    const int rpc = smooth_rows(sp, n, 256, (int)std::min<long long>(4096, nrows * n / (148 * 4)));
     const size_t smem = 2 * sizeof(float2) * (size_t)rpc * n;
     const float2* tw = twiddles(n);
     const long long grid = (nrows + rpc - 1) / rpc;

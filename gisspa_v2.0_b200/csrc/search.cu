@@ -587,6 +587,7 @@ TuneChoice autotune(Ctx& c, int epi, const float2* I, int W, const void* T, int 
         continue;
       }
       if (!correlate_variant_ok(l, v, epi)) continue;
+      if (epi == EPI_NONORM && v > 0) continue;  // one row kernel
       // (a pruned second sweep's few live pairs do not need the column shape tuned)
       const int n_av = (epi == EPI_CHUNK && args.skip.pairs) ? 1 : pass_a_variants(l);
       for (int av = 0; av < n_av; ++av) {
