@@ -185,7 +185,8 @@ __global__ void gen_map_kernel(const float2* __restrict__ X, CorrArgs a, int L) 
 // registers (336 = 7 6 8) instead of 2, 3, 4, 5 and 7 with table reads per point, multiplications
 // instead of divisions by run-time sizes, rows per CTA that fill its passes, and an intermediate
 // that both passes move in whole sectors took a top-K search of 1500 x 1401 pixels at window 336
-// (20 templates, 30 angles) from 59.1 to 35.0 ms.
+// (20 templates, 30 angles) from 59.1 to 35.0 ms; the first and last stages' own loads and stores,
+// accumulators in registers and launches of even size from there to 28.0.
 
 // Rows per CTA of gen_rows_kernel: even, a divisor of L, about 1280 pixels per CTA, and for
 // the chunk scans (EPI_CHUNK, EPI_NONORM) RB L a multiple of 256; 0 when no such RB exists.
@@ -210,48 +211,192 @@ __host__ __device__ constexpr int gen_rows_rb(int L, int epi) {
 __device__ __forceinline__ size_t gen_z_index(int p, int kx, int y, int L, int hz) {
   return (((size_t)p * (L >> 2) + (y >> 2)) * hz + kx) * 4 + (y & 3);
 }
-constexpr int kGenColPad = 4;  // the columns' stride in shared memory, beyond L: writes without bank conflicts
 
 // Column pass: rows gr = p (L/2+1) + kx of the launch's half-spectrum products
 // I[b0 + e][kx][.] conj(T[n0 + d][kx][.]) (p = e D + d), each inverse-transformed along ky in
-// shared memory: Z (gen_z_index).  rpc <= kGenMaxCols
+// shared memory: Z (gen_z_index).  The first stage reads its points from memory, the last writes
+// them there (four neighbouring butterflies fill a sector).  rpc <= kGenMaxCols
 constexpr int kGenMaxCols = 128;
 template <typename SPEC>
-__global__ void __launch_bounds__(256) gen_cols_kernel(const float2* __restrict__ I,
-                                                       const typename SPEC::T* __restrict__ T, int b0, int n0, int D,
-                                                       int L, unsigned div_l, int nrows, int rpc, SmoothPlan plan,
-                                                       const float2* __restrict__ tw, float2* __restrict__ Z) {
+__global__ void __launch_bounds__(256, 3) gen_cols_kernel(const float2* __restrict__ I,
+                                                          const typename SPEC::T* __restrict__ T, int b0, int n0,
+                                                          int D, int L, int nrows, int rpc, SmoothPlan plan,
+                                                          const float2* __restrict__ tw, float2* __restrict__ Z) {
   extern __shared__ float2 sm[];
-  __shared__ long long iof[kGenMaxCols], tof[kGenMaxCols];
-  __shared__ int zp[kGenMaxCols], zk[kGenMaxCols];
-  const int hz = L / 2 + 1, ld = L + kGenColPad;
+  __shared__ long long iof[kGenMaxCols], tof[kGenMaxCols], zof[kGenMaxCols];
+  const int hz = L / 2 + 1;
   const long long H = (long long)hz * L;
   const int row0 = blockIdx.x * rpc;
   const int rows_here = min(rpc, nrows - row0);
   float2* a = sm;
-  float2* b = sm + (size_t)rpc * ld;
+  float2* b = sm + (size_t)rpc * L;
   for (int r = threadIdx.x; r < rows_here; r += 256) {
     const int gr = row0 + r, p = gr / hz, kx = gr - p * hz, e = p / D, d = p - e * D;
     iof[r] = (b0 + e) * H + (long long)kx * L;
     tof[r] = (n0 + d) * H + (long long)kx * L;
-    zp[r] = p;
-    zk[r] = kx;
+    zof[r] = (long long)gen_z_index(p, kx, 0, L, hz);
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < rows_here * L; i += 256) {
-    const int r = fast_div(i, div_l), k = i - r * L;
-    a[r * ld + k] = cmulc(I[iof[r] + k], SPEC::load(T + tof[r] + k));
-  }
+  smooth_any<1>(plan, 0, rows_here, L, 1, tw,
+                [&](int r, int j, int m, auto& x) {
+                  constexpr int R = sizeof(x) / sizeof(float2);
+                  const float2* i = I + iof[r] + j;
+                  const typename SPEC::T* t = T + tof[r] + j;
+#pragma unroll
+                  for (int q = 0; q < R; ++q) x[q] = cmulc(__ldg(i + q * m), SPEC::load(t + q * m));
+                },
+                SmoothStore{a, L, 1});
   __syncthreads();
-  const float2* f = smooth_stages<1>(a, b, rows_here, L, ld, plan, tw);
-  const unsigned div_r = fast_div_mul(rows_here);
-  for (int i = threadIdx.x; i < rows_here * L; i += 256) {
-    const int j = i & 3, q = i >> 2, yb = fast_div(q, div_r), r = q - yb * rows_here, y = yb * 4 + j;
-    Z[gen_z_index(zp[r], zk[r], y, L, hz)] = f[r * ld + y];
+  const int last = plan.ns - 1, Ns = L / plan.r[last];
+  const float2* f = smooth_stages<1>(a, b, rows_here, L, L, plan, 1, last, plan.r[0], tw);
+  smooth_any<1>(plan, last, rows_here, L, Ns, tw, SmoothLoad{f, L}, [&](int r, int base, const auto& x) {
+    constexpr int R = sizeof(x) / sizeof(float2);
+    float2* o = Z + zof[r];
+#pragma unroll
+    for (int p = 0; p < R; ++p) {
+      const int y = base + p * Ns;
+      o[(y >> 2) * (4 * hz) + (y & 3)] = x[p];
+    }
+  });
+}
+
+// Where the row passes' threads load a template's Hermitian half rows: thread t < (256 / hr) hr
+// takes complex row r2 = t mod hr of the CTA's and columns k0 = t / hr, k0 + step, ...
+struct GenRowLoad {
+  int r2, k0, step, ya, yb;
+  __device__ __forceinline__ GenRowLoad(int t, int L, int Y0, int hr) {
+    step = 256 / hr;
+    k0 = t / hr;
+    r2 = t - k0 * hr;
+    if (k0 >= step) k0 = L;  // no columns
+    ya = Y0 + r2 + L / 2;
+    yb = ya + hr;
+    ya -= ya >= L ? L : 0;
+    yb -= yb >= L ? L : 0;
+  }
+  // X_r + i X_{r + hr} of pair p over all columns into row (row r2 of the template's rows)
+  __device__ __forceinline__ void run(const float2* __restrict__ Z, int p, int L, int hz, float2* row) const {
+    const float2* A = Z + gen_z_index(p, 0, ya, L, hz);
+    const float2* B = Z + gen_z_index(p, 0, yb, L, hz);
+#pragma unroll 4
+    for (int k = k0; k < hz; k += step) {
+      const float2 u = A[4 * k], v = B[4 * k];
+      row[k] = make_float2(u.x - v.y, u.y + v.x);
+      if (k > 0 && 2 * k < L) row[L - k] = make_float2(u.x + v.y, v.x - u.y);
+    }
+  }
+};
+
+// Row pass of EPI_SUM and EPI_TOPK: one CTA per (block of RB window rows, window of the launch), RB
+// / 2 complex rows (as gen_rows_kernel) of TB templates at a time.  The plan ends in a stage of 8
+// points, whose butterflies stay with their threads for all groups of templates: a thread keeps the
+// sums (and maxima) of its 16 pixels over every TB-th template in registers, and the TB threads of a
+// pixel meet in shared memory at the end.  RB / 2 L / 8 TB <= 256 threads.
+constexpr int kFold = 8;
+template <int EPI>
+__global__ void __launch_bounds__(256, EPI == EPI_TOPK ? 2 : 3)
+    gen_fold_kernel(const float2* __restrict__ Z, CorrArgs a, int L, int RB, int ld, int TB, SmoothPlan plan,
+                    const float2* __restrict__ tw) {
+  extern __shared__ float2 sm[];
+  constexpr bool TOPK = EPI == EPI_TOPK;
+  const int hz = L / 2 + 1, hr = RB / 2, t = threadIdx.x, m = L / kFold, per = hr * m;
+  const int e = blockIdx.y, Y0 = blockIdx.x * RB;
+  const long long L2 = (long long)L * L;
+  const float inv = 1.0f / (float)L2;
+  float2* buf0 = sm;  // TB templates x hr complex rows, row stride ld
+  float2* buf1 = sm + (size_t)TB * hr * ld;
+  const GenRowLoad rows(t, L, Y0, hr);
+  const int g = t / per, rem = t - g * per, r = rem / m, j = rem - r * m;  // this thread's butterflies
+  float s1[2][kFold], s2[2][kFold], best[TOPK ? 2 : 1][kFold];
+  unsigned arg[TOPK ? kFold : 1];  // template of the launch + 1 of the two pixels' maxima, 16 bits each
+#pragma unroll
+  for (int i = 0; i < kFold; ++i) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      s1[h][i] = s2[h][i] = 0.f;
+      if constexpr (TOPK) best[h][i] = -INFINITY;
+    }
+    if constexpr (TOPK) arg[i] = 0u;
+  }
+  for (int d0 = 0; d0 < a.D; d0 += TB) {
+    const int nd = min(TB, a.D - d0);
+    for (int q = 0; q < nd; ++q) rows.run(Z, e * a.D + d0 + q, L, hz, buf0 + (q * hr + rows.r2) * ld);
+    __syncthreads();
+    const float2* f = smooth_stages<1>(buf0, buf1, nd * hr, L, ld, plan, 0, plan.ns - 1, 1, tw);
+    if (g < nd) {
+      float2 x[kFold];
+      SmoothLoad{f, ld}(g * hr + r, j, m, x);
+      twiddle_powers<kFold, 1>(x, tw, j);
+      Dft<kFold, 1>::run(x);
+#pragma unroll
+      for (int i = 0; i < kFold; ++i) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float c = (h ? x[i].y : x[i].x) * inv;
+          s1[h][i] += c;
+          s2[h][i] = fmaf(c, c, s2[h][i]);
+          if constexpr (TOPK) {
+            if (c > best[h][i]) {
+              best[h][i] = c;
+              arg[i] = h ? (arg[i] & 0xFFFFu) | (unsigned)(d0 + g + 1) << 16 : (arg[i] & 0xFFFF0000u) | (d0 + g + 1);
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();  // the transform buffers are rewritten next
+  }
+  // the TB shares of every pixel, in order (one value of every thread at a time)
+  float* sh = reinterpret_cast<float*>(sm);
+  const int angle = a.angle_state ? a.angle_state->index : a.angle;
+  const size_t wpix = (size_t)(a.b0 + e) * L2;
+#pragma unroll
+  for (int i = 0; i < kFold; ++i) {
+    const int xc = j + i * m, ox = xc + L / 2 - (xc + L / 2 >= L ? L : 0);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      unsigned own = 0;
+      if constexpr (TOPK) own = h ? arg[i] >> 16 : arg[i] & 0xFFFFu;
+      sh[t] = s1[h][i];
+      sh[256 + t] = s2[h][i];
+      if constexpr (TOPK) {
+        sh[512 + t] = best[h][i];
+        sh[768 + t] = __uint_as_float(own);
+      }
+      __syncthreads();
+      if (t < per) {
+        float v1 = sh[t], v2 = sh[256 + t], b = 0.f;
+        unsigned w = own;
+        if constexpr (TOPK) b = best[h][i];
+        for (int q = 1; q < TB; ++q) {
+          const int o = t + q * per;
+          v1 += sh[o];
+          v2 += sh[256 + o];
+          if constexpr (TOPK) {
+            const float c = sh[512 + o];
+            const unsigned n = __float_as_uint(sh[768 + o]);
+            if (n && (c > b || (c == b && n < w))) {
+              b = c;
+              w = n;
+            }
+          }
+        }
+        const size_t pix = wpix + (size_t)(Y0 + r + h * hr) * L + ox;
+        atomicAdd(a.S1 + pix, (double)v1);
+        atomicAdd(a.S2 + pix, (double)v2);
+        if constexpr (TOPK) {
+          if (w) {
+            const unsigned id = (unsigned)(angle * a.nt_total + a.n0) + w - 1;
+            atomicMax(a.peak + pix, ((unsigned long long)float_key(b) << 32) | (unsigned)(0xFFFFFFFFu - id));
+          }
+        }
+      }
+      __syncthreads();
+    }
   }
 }
 
-// Row pass: one CTA per (block of RB window rows, window of the launch), over the launch's D
+// Row pass of the other epilogues: one CTA per (block of RB window rows, window of the launch), over the launch's D
 // templates.  Window (state) row Y0 + r is transform row (Y0 + r + L/2) mod L, and state
 // column ox is transform column (ox + L/2) mod L (zero lag at (L/2, L/2)).  Rows r and
 // r + RB/2 are real, so their Hermitian spectra X_r[k] (= Z[p][k][y] for k <= L/2,
@@ -280,22 +425,8 @@ __global__ void __launch_bounds__(256, 3) gen_rows_kernel(const float2* __restri
   const size_t wpix = (size_t)win * L2 + (size_t)Y0 * L;
   const float inv = 1.0f / (float)L2;
   const int angle = a.angle_state ? a.angle_state->index : a.angle;
-  const unsigned div_hr = fast_div_mul(hr), div_hz = fast_div_mul(hz);
-  float* s1 = reinterpret_cast<float*>(st);  // SUM / TOPK per-pixel accumulators
-  float* s2 = s1 + npix;
-  float* bst = s2 + npix;
-  int* barg = reinterpret_cast<int*>(bst + npix);
+  const GenRowLoad rows(t, L, Y0, hr);
   float2* ms = reinterpret_cast<float2*>(st);  // CHUNK: (mu, 1/sigma) of the CTA's pixels
-  if constexpr (EPI == EPI_SUM || EPI == EPI_TOPK) {
-    for (int q = t; q < npix; q += 256) {
-      s1[q] = 0.f;
-      s2[q] = 0.f;
-      if constexpr (EPI == EPI_TOPK) {
-        bst[q] = -INFINITY;
-        barg[q] = -1;
-      }
-    }
-  }
   if constexpr (EPI == EPI_CHUNK)
     for (int q = t; q < npix; q += 256) ms[q] = a.musig[wpix + q];
   // pixel q's place in a template's transformed rows (complex row, column) and which part
@@ -308,50 +439,10 @@ __global__ void __launch_bounds__(256, 3) gen_rows_kernel(const float2* __restri
   for (int d0 = 0; d0 < a.D; d0 += TB) {
     const int nd = min(TB, a.D - d0);
     if (EPI == EPI_CHUNK && t == 0) hits = 0u;
-    for (int idx = t; idx < nd * hr * hz; idx += 256) {
-      const int q = fast_div(idx, div_hr), r2 = idx - q * hr, g = fast_div(q, div_hz), k = q - g * hz;
-      int ya = Y0 + r2 + L / 2, yb = ya + hr;
-      ya -= ya >= L ? L : 0;
-      yb -= yb >= L ? L : 0;
-      const int p = e * a.D + d0 + g;
-      const float2 A = Z[gen_z_index(p, k, ya, L, hz)], B = Z[gen_z_index(p, k, yb, L, hz)];
-      float2* row = buf0 + (g * hr + r2) * ld;
-      row[k] = make_float2(A.x - B.y, A.y + B.x);
-      if (k > 0 && 2 * k < L) row[L - k] = make_float2(A.x + B.y, B.x - A.y);
-    }
+    for (int q = 0; q < nd; ++q) rows.run(Z, e * a.D + d0 + q, L, hz, buf0 + (q * hr + rows.r2) * ld);
     __syncthreads();
-    const float2* fg = smooth_stages<1>(buf0, buf1, nd * hr, L, ld, plan, tw);
+    const float2* fg = smooth_stages<1>(buf0, buf1, nd * hr, L, ld, plan, 0, plan.ns, 1, tw);
 
-    // each pixel folds the group's templates in order, as the one-at-a-time sweep would
-    if constexpr (EPI == EPI_SUM || EPI == EPI_TOPK) {
-      for (int q = t; q < npix; q += 256) {
-        bool up;
-        const float2* f = fg + place(q, up);
-        float v1 = s1[q], v2 = s2[q], b = 0.f;
-        int arg = -1;
-        if constexpr (EPI == EPI_TOPK) b = bst[q];
-        for (int g = 0; g < nd; ++g) {
-          const float2 w = f[g * hr * ld];
-          const float c = (up ? w.y : w.x) * inv;
-          v1 += c;
-          v2 = fmaf(c, c, v2);
-          if constexpr (EPI == EPI_TOPK) {
-            if (c > b) {
-              b = c;
-              arg = d0 + g;
-            }
-          }
-        }
-        s1[q] = v1;
-        s2[q] = v2;
-        if constexpr (EPI == EPI_TOPK) {
-          if (arg >= 0) {
-            bst[q] = b;
-            barg[q] = angle * a.nt_total + a.n0 + arg;
-          }
-        }
-      }
-    }
     if constexpr (EPI == EPI_CHUNK) {
       unsigned hit = 0;
       for (int q = t; q < npix; q += 256) {
@@ -471,18 +562,6 @@ __global__ void __launch_bounds__(256, 3) gen_rows_kernel(const float2* __restri
     }
     __syncthreads();  // the transform buffers are rewritten next
   }
-
-  if constexpr (EPI == EPI_SUM || EPI == EPI_TOPK) {
-    for (int q = t; q < npix; q += 256) {
-      atomicAdd(a.S1 + wpix + q, (double)s1[q]);
-      atomicAdd(a.S2 + wpix + q, (double)s2[q]);
-      if constexpr (EPI == EPI_TOPK) {
-        if (barg[q] >= 0)
-          atomicMax(a.peak + wpix + q,
-                    ((unsigned long long)float_key(bst[q]) << 32) | (unsigned)(0xFFFFFFFFu - (unsigned)barg[q]));
-      }
-    }
-  }
 }
 
 // Row stride in shared memory: the loads write hr rows of a column at a time, 16 / hr columns per
@@ -492,13 +571,13 @@ int gen_rows_ld(int L, int RB) { return L + std::max(1, 16 / (RB / 2)); }
 size_t gen_rows_smem(int L, int RB, int epi, int tb) {
   const size_t ld = gen_rows_ld(L, RB), npix = (size_t)RB * L, nch = npix / 256;
   size_t b = sizeof(float2) * tb * RB * ld + sizeof(unsigned long long) * nch * 8 + sizeof(double) * 16;
-  if (epi == EPI_SUM || epi == EPI_TOPK) b += 16 * npix;
+  if (epi == EPI_SUM || epi == EPI_TOPK) b = std::max<size_t>(sizeof(float2) * tb * RB * ld, 16 * 256);
   if (epi == EPI_CHUNK) b += sizeof(float2) * npix;
   return b;
 }
 
 constexpr size_t kGenSmemMax = 200 * 1024;
-constexpr int kGenColPoints = 5632;  // per CTA of the column pass (88 KB: two CTAs per SM)
+constexpr int kGenColPoints = 4352;  // per CTA of the column pass (68 KB: three CTAs per SM)
 
 // Templates per transform pass of gen_rows_kernel: as fill its CTA's passes best (smooth_rows), three
 // CTAs per SM where one template's rows leave room for that.
@@ -507,6 +586,8 @@ int gen_rows_tb(int L, int RB, int epi, const SmoothPlan& plan) {
   const size_t one = gen_rows_smem(L, RB, epi, 1), two = gen_rows_smem(L, RB, epi, 2);
   const size_t room = kGenSmemMax / 3 > one ? kGenSmemMax / 3 - one : 0;
   const int tb = std::min<long long>(kGenTB, 1 + room / (two - one));
+  if (epi == EPI_SUM || epi == EPI_TOPK)  // every thread of the last stage has its own butterfly
+    return std::max(1, std::min(tb, 256 / (RB / 2 * L / kFold)));
   return smooth_rows(plan, L, 256, tb * (RB / 2) * L, RB / 2) / (RB / 2);
 }
 
@@ -527,7 +608,8 @@ auto gen_kernel(size_t smem) {
 bool generic_fused(int L, int epi) {
   if (L > kSmoothMax || smooth_plan(L).ns == 0) return false;
   const int rb = gen_rows_rb(L, epi);
-  return rb > 0 && gen_rows_smem(L, rb, epi, 1) <= kGenSmemMax && (size_t)2 * sizeof(float2) * (L + kGenColPad) <= kGenSmemMax;
+  if ((epi == EPI_SUM || epi == EPI_TOPK) && rb / 2 * L / kFold > 256) return false;
+  return rb > 0 && gen_rows_smem(L, rb, epi, 1) <= kGenSmemMax && (size_t)2 * sizeof(float2) * L <= kGenSmemMax;
 }
 
 bool correlate_fast(int L) { return L == 256 || L == 320 || L == 512 || L == 1024; }
@@ -546,10 +628,10 @@ void correlate_generic(const CorrLaunch& cl, const float2* I, const void* T, con
     const unsigned div_l = fast_div_mul(L);
     const int nrows = P * (L / 2 + 1);
     const int rpc = std::min(kGenMaxCols, smooth_rows(plan, L, 256, kGenColPoints));
-    const size_t smc = 2 * sizeof(float2) * (size_t)rpc * (L + kGenColPad);
+    const size_t smc = 2 * sizeof(float2) * (size_t)rpc * L;
     const unsigned gc = (unsigned)ceil_div(nrows, rpc);
     auto cols = [&](auto kernel, const auto* t) {
-      kernel<<<gc, 256, smc, s>>>(I, t, a.b0, a.n0, cl.D, L, div_l, nrows, rpc, plan, tw, z);
+      kernel<<<gc, 256, smc, s>>>(I, t, a.b0, a.n0, cl.D, L, nrows, rpc, plan, tw, z);
     };
     switch (cl.spec) {
       case GISSPA_SPEC_FP32: cols(gen_kernel<gen_cols_kernel<SpecFp32>>(smc), static_cast<const float2*>(T)); break;
@@ -562,13 +644,16 @@ void correlate_generic(const CorrLaunch& cl, const float2* I, const void* T, con
     GISSPA_LAUNCH_CHECK();
     if (ev) GISSPA_CUDA(cudaEventRecord(ev[1], s));
     const int rb = gen_rows_rb(L, cl.epi), ld = gen_rows_ld(L, rb);
-    const int tb = std::min(gen_rows_tb(L, rb, cl.epi, plan), cl.D);
+    const int most = gen_rows_tb(L, rb, cl.epi, plan), tb = ceil_div(cl.D, ceil_div(cl.D, most));
     const size_t smr = gen_rows_smem(L, rb, cl.epi, tb);
     const dim3 gr((unsigned)(L / rb), (unsigned)cl.E);
     auto rows = [&](auto kernel) { kernel<<<gr, 256, smr, s>>>(z, a, L, div_l, rb, ld, tb, plan, tw); };
+    auto fold = [&](auto kernel) {
+      kernel<<<gr, 256, smr, s>>>(z, a, L, rb, ld, tb, smooth_plan(L, kFold), tw);
+    };
     switch (cl.epi) {
-      case EPI_SUM: rows(gen_kernel<gen_rows_kernel<EPI_SUM>>(smr)); break;
-      case EPI_TOPK: rows(gen_kernel<gen_rows_kernel<EPI_TOPK>>(smr)); break;
+      case EPI_SUM: fold(gen_kernel<gen_fold_kernel<EPI_SUM>>(smr)); break;
+      case EPI_TOPK: fold(gen_kernel<gen_fold_kernel<EPI_TOPK>>(smr)); break;
       case EPI_CHUNK: rows(gen_kernel<gen_rows_kernel<EPI_CHUNK>>(smr)); break;
       case EPI_NONORM: rows(gen_kernel<gen_rows_kernel<EPI_NONORM>>(smr)); break;
       case EPI_MAP: rows(gen_kernel<gen_rows_kernel<EPI_MAP>>(smr)); break;

@@ -113,7 +113,7 @@ __global__ void fft_smooth_rows_kernel(float2* __restrict__ data, long long nrow
   const int total = rows_here * n;
   for (int i = threadIdx.x; i < total; i += blockDim.x) a[i] = base[i];
   __syncthreads();
-  a = smooth_stages<SIGN>(a, b, rows_here, n, n, plan, tw);
+  a = smooth_stages<SIGN>(a, b, rows_here, n, n, plan, 0, plan.ns, 1, tw);
   for (int i = threadIdx.x; i < total; i += blockDim.x) base[i] = cscale(a[i], scale);
 }
 
@@ -206,7 +206,20 @@ bool smooth_split(int n, int ns, int top, int* r) {
 }
 }  // namespace
 
-SmoothPlan smooth_plan(int n) {
+SmoothPlan smooth_plan(int n, int last) {
+  if (last) {
+    SmoothPlan p = smooth_plan(n / last);
+    if (!p.ns) return p;
+    int Ns = 1;
+    for (int s = 0; s < p.ns; ++s) {
+      p.div_m[s] = fast_div_mul(n / p.r[s]);
+      Ns *= p.r[s];
+    }
+    p.div_m[p.ns] = fast_div_mul(Ns);
+    p.div_ns[p.ns] = fast_div_mul(Ns);
+    p.r[p.ns++] = last;
+    return p;
+  }
   SmoothPlan p;
   int rest = n;
   for (int f : {2, 3, 5, 7})

@@ -70,7 +70,7 @@ class DevBuf {
 // first stage writes its outputs R apart, in distinct banks for odd R.
 constexpr int kSmoothRadices[] = {2, 3, 4, 5, 6, 7, 8, 10, 12, 14, 15, 16};
 struct SmoothPlan {
-  static constexpr int kMax = 13;  // radices of 2^13
+  static constexpr int kMax = 14;  // radices of 2^13 and one more
   int ns = 0;
   int r[kMax] = {};
   unsigned div_m[kMax] = {}, div_ns[kMax] = {};  // fast_div of n / r and of the radices before
@@ -80,7 +80,8 @@ __host__ __device__ constexpr unsigned fast_div_mul(unsigned d) {
   return d > 1 ? (unsigned)(((1ull << 32) + d - 1) / d) : 0;
 }
 __device__ __forceinline__ int fast_div(int i, unsigned mul) { return mul ? (int)__umulhi((unsigned)i, mul) : i; }
-SmoothPlan smooth_plan(int n);
+// last: a divisor of n to end with (0: any).
+SmoothPlan smooth_plan(int n, int last = 0);
 // Rows of length n per CTA of `threads`, a multiple of `step`, of at most max_points points (or
 // `step`): the count whose butterflies fill the CTA's passes best.
 int smooth_rows(const SmoothPlan& plan, int n, int threads, int max_points, int step = 1);

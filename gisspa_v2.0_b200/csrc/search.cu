@@ -462,8 +462,15 @@ void choose_batches(const gisspa_config& cfg, int l, int W, int nt, int& D, int&
   // twice the CTAs of 8 (4096^2 at L = 320: 20.0 against 21.7 s per micrograph)
   E = cfg.window_batch > 0 ? cfg.window_batch : (!correlate_fast(l) ? 16 : (l >= 1024 ? 4 : 8));
   E = std::max(1, std::min(E, W));
+  // (their launches evened out)
+  auto even = [](int n, int per) { return ceil_div(n, ceil_div(n, per)); };
+  if (cfg.window_batch <= 0 && !correlate_fast(l)) E = even(W, E);
   D = cfg.template_batch > 0 ? cfg.template_batch : (int)std::max(1LL, budget / per_pair / E);
   D = std::max(1, std::min(D, nt));
+  if (!correlate_fast(l)) {
+    D = std::min(D, 65534);  // (the generic row pass keeps a launch's template in 16 bits)
+    if (cfg.template_batch <= 0) D = even(nt, D);
+  }
 }
 
 // The pair engine's launch sequence over `batches` (first window, first template, windows,
