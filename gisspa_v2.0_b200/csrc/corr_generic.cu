@@ -186,7 +186,8 @@ __global__ void gen_map_kernel(const float2* __restrict__ X, CorrArgs a, int L) 
 // instead of divisions by run-time sizes, rows per CTA that fill its passes, and an intermediate
 // that both passes move in whole sectors took a top-K search of 1500 x 1401 pixels at window 336
 // (20 templates, 30 angles) from 59.1 to 35.0 ms; the first and last stages' own loads and stores,
-// accumulators in registers and launches of even size from there to 28.0.
+// accumulators in registers, groups of warps with their own barriers and fewer, even launches from
+// there to 23.8.
 
 // Rows per CTA of gen_rows_kernel: even, a divisor of L, about 1280 pixels per CTA, and for
 // the chunk scans (EPI_CHUNK, EPI_NONORM) RB L a multiple of 256; 0 when no such RB exists.
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(256, 3) gen_cols_kernel(const float2* __restri
     zof[r] = (long long)gen_z_index(p, kx, 0, L, hz);
   }
   __syncthreads();
-  smooth_any<1>(plan, 0, rows_here, L, 1, tw,
+  smooth_any<1>(CtaTeam{}, plan, 0, rows_here, L, 1, tw,
                 [&](int r, int j, int m, auto& x) {
                   constexpr int R = sizeof(x) / sizeof(float2);
                   const float2* i = I + iof[r] + j;
@@ -248,8 +249,8 @@ __global__ void __launch_bounds__(256, 3) gen_cols_kernel(const float2* __restri
                 SmoothStore{a, L, 1});
   __syncthreads();
   const int last = plan.ns - 1, Ns = L / plan.r[last];
-  const float2* f = smooth_stages<1>(a, b, rows_here, L, L, plan, 1, last, plan.r[0], tw);
-  smooth_any<1>(plan, last, rows_here, L, Ns, tw, SmoothLoad{f, L}, [&](int r, int base, const auto& x) {
+  const float2* f = smooth_stages<1>(CtaTeam{}, a, b, rows_here, L, L, plan, 1, last, plan.r[0], tw);
+  smooth_any<1>(CtaTeam{}, plan, last, rows_here, L, Ns, tw, SmoothLoad{f, L}, [&](int r, int base, const auto& x) {
     constexpr int R = sizeof(x) / sizeof(float2);
     float2* o = Z + zof[r];
 #pragma unroll
@@ -260,12 +261,13 @@ __global__ void __launch_bounds__(256, 3) gen_cols_kernel(const float2* __restri
   });
 }
 
-// Where the row passes' threads load a template's Hermitian half rows: thread t < (256 / hr) hr
-// takes complex row r2 = t mod hr of the CTA's and columns k0 = t / hr, k0 + step, ...
+// Where the row passes' threads load a template's Hermitian half rows: of a team of `threads`, thread
+// t < (threads / hr) hr takes complex row r2 = t mod hr of the CTA's and columns k0 = t / hr, k0 +
+// step, ...  (hr <= threads)
 struct GenRowLoad {
   int r2, k0, step, ya, yb;
-  __device__ __forceinline__ GenRowLoad(int t, int L, int Y0, int hr) {
-    step = 256 / hr;
+  __device__ __forceinline__ GenRowLoad(int t, int threads, int L, int Y0, int hr) {
+    step = threads / hr;
     k0 = t / hr;
     r2 = t - k0 * hr;
     if (k0 >= step) k0 = L;  // no columns
@@ -288,25 +290,30 @@ struct GenRowLoad {
 };
 
 // Row pass of EPI_SUM and EPI_TOPK: one CTA per (block of RB window rows, window of the launch), RB
-// / 2 complex rows (as gen_rows_kernel) of TB templates at a time.  The plan ends in a stage of 8
-// points, whose butterflies stay with their threads for all groups of templates: a thread keeps the
-// sums (and maxima) of its 16 pixels over every TB-th template in registers, and the TB threads of a
-// pixel meet in shared memory at the end.  RB / 2 L / 8 TB <= 256 threads.
-constexpr int kFold = 8;
+// / 2 complex rows (as gen_rows_kernel).  The CTA's groups of warps take every `groups`-th template
+// of the launch, each with its own buffers and barrier.  The plan ends in a stage of 8 points, whose
+// butterflies stay with their threads for all templates: a thread keeps the sums (and maxima) of its
+// 16 pixels in registers, and the groups meet in shared memory at the end.
+constexpr int kFold = 8, kFoldThreads = 512;
+// Warps of a group: a thread for each of the last stage's butterflies
+__host__ __device__ constexpr int gen_fold_warps(int L, int RB) { return (RB / 2 * L / kFold + 31) / 32; }
 template <int EPI>
-__global__ void __launch_bounds__(256, EPI == EPI_TOPK ? 2 : 3)
-    gen_fold_kernel(const float2* __restrict__ Z, CorrArgs a, int L, int RB, int ld, int TB, SmoothPlan plan,
+__global__ void __launch_bounds__(kFoldThreads)
+    gen_fold_kernel(const float2* __restrict__ Z, CorrArgs a, int L, int RB, int ld, int groups, SmoothPlan plan,
                     const float2* __restrict__ tw) {
   extern __shared__ float2 sm[];
   constexpr bool TOPK = EPI == EPI_TOPK;
-  const int hz = L / 2 + 1, hr = RB / 2, t = threadIdx.x, m = L / kFold, per = hr * m;
-  const int e = blockIdx.y, Y0 = blockIdx.x * RB;
+  constexpr int NV = TOPK ? 4 : 2;  // values per pixel
+  const int hz = L / 2 + 1, hr = RB / 2, m = L / kFold, per = hr * m, threads = 32 * gen_fold_warps(L, RB);
+  const int e = blockIdx.y, Y0 = blockIdx.x * RB, g = threadIdx.x / threads;
   const long long L2 = (long long)L * L;
   const float inv = 1.0f / (float)L2;
-  float2* buf0 = sm;  // TB templates x hr complex rows, row stride ld
-  float2* buf1 = sm + (size_t)TB * hr * ld;
-  const GenRowLoad rows(t, L, Y0, hr);
-  const int g = t / per, rem = t - g * per, r = rem / m, j = rem - r * m;  // this thread's butterflies
+  const WarpsTeam team{g, threads};
+  const int t = team.id(), r = t / m, j = t - r * m;  // this thread's butterfly
+  const bool own = t < per;
+  float2* buf0 = sm + (size_t)g * 2 * hr * ld;  // hr complex rows, row stride ld
+  float2* buf1 = buf0 + (size_t)hr * ld;
+  const GenRowLoad rows(t, threads, L, Y0, hr);
   float s1[2][kFold], s2[2][kFold], best[TOPK ? 2 : 1][kFold];
   unsigned arg[TOPK ? kFold : 1];  // template of the launch + 1 of the two pixels' maxima, 16 bits each
 #pragma unroll
@@ -318,14 +325,13 @@ __global__ void __launch_bounds__(256, EPI == EPI_TOPK ? 2 : 3)
     }
     if constexpr (TOPK) arg[i] = 0u;
   }
-  for (int d0 = 0; d0 < a.D; d0 += TB) {
-    const int nd = min(TB, a.D - d0);
-    for (int q = 0; q < nd; ++q) rows.run(Z, e * a.D + d0 + q, L, hz, buf0 + (q * hr + rows.r2) * ld);
-    __syncthreads();
-    const float2* f = smooth_stages<1>(buf0, buf1, nd * hr, L, ld, plan, 0, plan.ns - 1, 1, tw);
-    if (g < nd) {
+  for (int d = g; d < a.D; d += groups) {
+    rows.run(Z, e * a.D + d, L, hz, buf0 + rows.r2 * ld);
+    team.sync();
+    const float2* f = smooth_stages<1>(team, buf0, buf1, hr, L, ld, plan, 0, plan.ns - 1, 1, tw);
+    if (own) {
       float2 x[kFold];
-      SmoothLoad{f, ld}(g * hr + r, j, m, x);
+      SmoothLoad{f, ld}(r, j, m, x);
       twiddle_powers<kFold, 1>(x, tw, j);
       Dft<kFold, 1>::run(x);
 #pragma unroll
@@ -338,60 +344,61 @@ __global__ void __launch_bounds__(256, EPI == EPI_TOPK ? 2 : 3)
           if constexpr (TOPK) {
             if (c > best[h][i]) {
               best[h][i] = c;
-              arg[i] = h ? (arg[i] & 0xFFFFu) | (unsigned)(d0 + g + 1) << 16 : (arg[i] & 0xFFFF0000u) | (d0 + g + 1);
+              arg[i] = h ? (arg[i] & 0xFFFFu) | (unsigned)(d + 1) << 16 : (arg[i] & 0xFFFF0000u) | (unsigned)(d + 1);
             }
           }
         }
       }
     }
-    __syncthreads();  // the transform buffers are rewritten next
+    team.sync();  // the buffers are rewritten next
   }
-  // the TB shares of every pixel, in order (one value of every thread at a time)
-  float* sh = reinterpret_cast<float*>(sm);
-  const int angle = a.angle_state ? a.angle_state->index : a.angle;
+  // every pixel's shares, in the groups' order; group g takes every groups-th of the 8 columns
+  float* sh = reinterpret_cast<float*>(sm);  // [kFold][NV][groups][per]
+  const int angle = a.angle_state ? a.angle_state->index : a.angle, all = groups * per;
   const size_t wpix = (size_t)(a.b0 + e) * L2;
 #pragma unroll
-  for (int i = 0; i < kFold; ++i) {
-    const int xc = j + i * m, ox = xc + L / 2 - (xc + L / 2 >= L ? L : 0);
+  for (int h = 0; h < 2; ++h) {
+    __syncthreads();
+    if (own) {
+      float* o = sh + g * per + t;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      unsigned own = 0;
-      if constexpr (TOPK) own = h ? arg[i] >> 16 : arg[i] & 0xFFFFu;
-      sh[t] = s1[h][i];
-      sh[256 + t] = s2[h][i];
-      if constexpr (TOPK) {
-        sh[512 + t] = best[h][i];
-        sh[768 + t] = __uint_as_float(own);
-      }
-      __syncthreads();
-      if (t < per) {
-        float v1 = sh[t], v2 = sh[256 + t], b = 0.f;
-        unsigned w = own;
-        if constexpr (TOPK) b = best[h][i];
-        for (int q = 1; q < TB; ++q) {
-          const int o = t + q * per;
-          v1 += sh[o];
-          v2 += sh[256 + o];
-          if constexpr (TOPK) {
-            const float c = sh[512 + o];
-            const unsigned n = __float_as_uint(sh[768 + o]);
-            if (n && (c > b || (c == b && n < w))) {
-              b = c;
-              w = n;
-            }
-          }
-        }
-        const size_t pix = wpix + (size_t)(Y0 + r + h * hr) * L + ox;
-        atomicAdd(a.S1 + pix, (double)v1);
-        atomicAdd(a.S2 + pix, (double)v2);
+      for (int i = 0; i < kFold; ++i) {
+        o[(NV * i) * all] = s1[h][i];
+        o[(NV * i + 1) * all] = s2[h][i];
         if constexpr (TOPK) {
-          if (w) {
-            const unsigned id = (unsigned)(angle * a.nt_total + a.n0) + w - 1;
-            atomicMax(a.peak + pix, ((unsigned long long)float_key(b) << 32) | (unsigned)(0xFFFFFFFFu - id));
+          o[(NV * i + 2) * all] = best[h][i];
+          o[(NV * i + 3) * all] = __uint_as_float(h ? arg[i] >> 16 : arg[i] & 0xFFFFu);
+        }
+      }
+    }
+    __syncthreads();
+    if (!own) continue;
+    for (int i = g; i < kFold; i += groups) {
+      const float* o = sh + (size_t)NV * i * all + t;
+      float v1 = 0.f, v2 = 0.f, b = -INFINITY;
+      unsigned w = 0;
+      for (int q = 0; q < groups; ++q, o += per) {
+        v1 += o[0];
+        v2 += o[all];
+        if constexpr (TOPK) {
+          const float c = o[2 * all];
+          const unsigned n = __float_as_uint(o[3 * all]);
+          if (n && (!w || c > b || (c == b && n < w))) {
+            b = c;
+            w = n;
           }
         }
       }
-      __syncthreads();
+      const int xc = j + i * m, ox = xc + L / 2 - (xc + L / 2 >= L ? L : 0);
+      const size_t pix = wpix + (size_t)(Y0 + r + h * hr) * L + ox;
+      atomicAdd(a.S1 + pix, (double)v1);
+      atomicAdd(a.S2 + pix, (double)v2);
+      if constexpr (TOPK) {
+        if (w) {
+          const unsigned id = (unsigned)(angle * a.nt_total + a.n0) + w - 1;
+          atomicMax(a.peak + pix, ((unsigned long long)float_key(b) << 32) | (unsigned)(0xFFFFFFFFu - id));
+        }
+      }
     }
   }
 }
@@ -425,7 +432,7 @@ __global__ void __launch_bounds__(256, 3) gen_rows_kernel(const float2* __restri
   const size_t wpix = (size_t)win * L2 + (size_t)Y0 * L;
   const float inv = 1.0f / (float)L2;
   const int angle = a.angle_state ? a.angle_state->index : a.angle;
-  const GenRowLoad rows(t, L, Y0, hr);
+  const GenRowLoad rows(t, 256, L, Y0, hr);
   float2* ms = reinterpret_cast<float2*>(st);  // CHUNK: (mu, 1/sigma) of the CTA's pixels
   if constexpr (EPI == EPI_CHUNK)
     for (int q = t; q < npix; q += 256) ms[q] = a.musig[wpix + q];
@@ -441,7 +448,7 @@ __global__ void __launch_bounds__(256, 3) gen_rows_kernel(const float2* __restri
     if (EPI == EPI_CHUNK && t == 0) hits = 0u;
     for (int q = 0; q < nd; ++q) rows.run(Z, e * a.D + d0 + q, L, hz, buf0 + (q * hr + rows.r2) * ld);
     __syncthreads();
-    const float2* fg = smooth_stages<1>(buf0, buf1, nd * hr, L, ld, plan, 0, plan.ns, 1, tw);
+    const float2* fg = smooth_stages<1>(CtaTeam{}, buf0, buf1, nd * hr, L, ld, plan, 0, plan.ns, 1, tw);
 
     if constexpr (EPI == EPI_CHUNK) {
       unsigned hit = 0;
@@ -571,7 +578,8 @@ int gen_rows_ld(int L, int RB) { return L + std::max(1, 16 / (RB / 2)); }
 size_t gen_rows_smem(int L, int RB, int epi, int tb) {
   const size_t ld = gen_rows_ld(L, RB), npix = (size_t)RB * L, nch = npix / 256;
   size_t b = sizeof(float2) * tb * RB * ld + sizeof(unsigned long long) * nch * 8 + sizeof(double) * 16;
-  if (epi == EPI_SUM || epi == EPI_TOPK) b = std::max<size_t>(sizeof(float2) * tb * RB * ld, 16 * 256);
+  if (epi == EPI_SUM || epi == EPI_TOPK)  // the groups' buffers, then their pixels' values
+    b = std::max<size_t>(sizeof(float2) * tb * RB * ld, sizeof(float) * (epi == EPI_TOPK ? 4 : 2) * tb * RB / 2 * L);
   if (epi == EPI_CHUNK) b += sizeof(float2) * npix;
   return b;
 }
@@ -586,8 +594,7 @@ int gen_rows_tb(int L, int RB, int epi, const SmoothPlan& plan) {
   const size_t one = gen_rows_smem(L, RB, epi, 1), two = gen_rows_smem(L, RB, epi, 2);
   const size_t room = kGenSmemMax / 3 > one ? kGenSmemMax / 3 - one : 0;
   const int tb = std::min<long long>(kGenTB, 1 + room / (two - one));
-  if (epi == EPI_SUM || epi == EPI_TOPK)  // every thread of the last stage has its own butterfly
-    return std::max(1, std::min(tb, 256 / (RB / 2 * L / kFold)));
+  if (epi == EPI_SUM || epi == EPI_TOPK) return std::max(1, std::min({tb, kFoldThreads / 32 / gen_fold_warps(L, RB), 15}));
   return smooth_rows(plan, L, 256, tb * (RB / 2) * L, RB / 2) / (RB / 2);
 }
 
@@ -608,7 +615,7 @@ auto gen_kernel(size_t smem) {
 bool generic_fused(int L, int epi) {
   if (L > kSmoothMax || smooth_plan(L).ns == 0) return false;
   const int rb = gen_rows_rb(L, epi);
-  if ((epi == EPI_SUM || epi == EPI_TOPK) && rb / 2 * L / kFold > 256) return false;
+  if ((epi == EPI_SUM || epi == EPI_TOPK) && gen_fold_warps(L, rb) * 32 > kFoldThreads) return false;
   return rb > 0 && gen_rows_smem(L, rb, epi, 1) <= kGenSmemMax && (size_t)2 * sizeof(float2) * L <= kGenSmemMax;
 }
 
@@ -649,7 +656,7 @@ void correlate_generic(const CorrLaunch& cl, const float2* I, const void* T, con
     const dim3 gr((unsigned)(L / rb), (unsigned)cl.E);
     auto rows = [&](auto kernel) { kernel<<<gr, 256, smr, s>>>(z, a, L, div_l, rb, ld, tb, plan, tw); };
     auto fold = [&](auto kernel) {
-      kernel<<<gr, 256, smr, s>>>(z, a, L, rb, ld, tb, smooth_plan(L, kFold), tw);
+      kernel<<<gr, 32 * tb * gen_fold_warps(L, rb), smr, s>>>(z, a, L, rb, ld, tb, smooth_plan(L, kFold), tw);
     };
     switch (cl.epi) {
       case EPI_SUM: fold(gen_kernel<gen_fold_kernel<EPI_SUM>>(smr)); break;

@@ -113,7 +113,7 @@ __global__ void fft_smooth_rows_kernel(float2* __restrict__ data, long long nrow
   const int total = rows_here * n;
   for (int i = threadIdx.x; i < total; i += blockDim.x) a[i] = base[i];
   __syncthreads();
-  a = smooth_stages<SIGN>(a, b, rows_here, n, n, plan, 0, plan.ns, 1, tw);
+  a = smooth_stages<SIGN>(CtaTeam{}, a, b, rows_here, n, n, plan, 0, plan.ns, 1, tw);
   for (int i = threadIdx.x; i < total; i += blockDim.x) base[i] = cscale(a[i], scale);
 }
 

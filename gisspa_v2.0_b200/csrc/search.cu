@@ -457,7 +457,7 @@ void template_spectra_listed(Ctx& c, float theta, const std::vector<int>& list) 
 
 void choose_batches(const gisspa_config& cfg, int l, int W, int nt, int& D, int& E) {
   const long long per_pair = (long long)(l / 2) * l * (long long)sizeof(float2);
-  const long long budget = 64LL << 20;
+  const long long budget = (correlate_fast(l) ? 64LL : 128LL) << 20;
   // window sizes without hand-tuned kernels: 16 windows per launch give the generic row kernel
   // twice the CTAs of 8 (4096^2 at L = 320: 20.0 against 21.7 s per micrograph)
   E = cfg.window_batch > 0 ? cfg.window_batch : (!correlate_fast(l) ? 16 : (l >= 1024 ? 4 : 8));
