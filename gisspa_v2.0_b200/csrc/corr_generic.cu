@@ -594,7 +594,7 @@ int gen_rows_tb(int L, int RB, int epi, const SmoothPlan& plan) {
   const size_t one = gen_rows_smem(L, RB, epi, 1), two = gen_rows_smem(L, RB, epi, 2);
   const size_t room = kGenSmemMax / 3 > one ? kGenSmemMax / 3 - one : 0;
   const int tb = std::min<long long>(kGenTB, 1 + room / (two - one));
-  if (epi == EPI_SUM || epi == EPI_TOPK) return std::max(1, std::min({tb, kFoldThreads / 32 / gen_fold_warps(L, RB), 15}));
+  if (epi == EPI_SUM || epi == EPI_TOPK) return std::max(1, std::min(std::min(tb, 15), kFoldThreads / 32 / gen_fold_warps(L, RB)));  // (15 barriers)
   return smooth_rows(plan, L, 256, tb * (RB / 2) * L, RB / 2) / (RB / 2);
 }
 
