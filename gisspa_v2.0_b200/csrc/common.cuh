@@ -210,6 +210,24 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned by
                "l"(src), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
+// Stores whose lines L2 should keep before others.
+__device__ __forceinline__ unsigned long long l2_keep_policy() {
+  unsigned long long p;
+  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+__device__ __forceinline__ void store_hint(float4* p, float4 v, unsigned long long policy) {
+  asm volatile("st.global.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z),
+               "f"(v.w), "l"(policy)
+               : "memory");
+}
+// Gives up the contents of `bytes` (a multiple of 128) from p (128-byte aligned): data that has been
+// read for the last time and lies in L2 need not be written back to DRAM.  Thread `id` of `threads`.
+__device__ __forceinline__ void discard_lines(const void* p, int bytes, int id, int threads) {
+  const char* c = static_cast<const char*>(p);
+  for (int i = id * 128; i < bytes; i += threads * 128)
+    asm volatile("discard.global.L2 [%0], 128;" ::"l"(c + i) : "memory");
+}
 // Bounded wait for the phase with the given parity: gives up after ~max_cycles SM
 // clock cycles (or 2^24 polls) and returns false.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, long long max_cycles) {

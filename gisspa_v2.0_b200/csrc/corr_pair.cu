@@ -19,6 +19,7 @@
 // a Q of 32 MB that stays in L2 0.26), the row pass by latency at 12 warps per SM (61 % of
 // issue slots; 552 instructions per row and template pair against 1090).
 #include <algorithm>
+#include <cfloat>
 
 #include "../../include/gisspa.h"
 #include "correlate.cuh"
@@ -72,7 +73,8 @@ __global__ void __launch_bounds__(col_threads<L, NC>(), MINB)
   griddep_launch_dependents();
   if (!chained) griddep_wait();  // the spectra may come from the kernel just before
   const int c0 = blockIdx.x * NC, tid = threadIdx.x;
-  const int p = blockIdx.y, e = p / DP, d = p - e * DP;
+  // all windows of a template pair, then the next pair: the row pass starts with the last ones
+  const int E = gridDim.y / DP, d = blockIdx.y / E, e = blockIdx.y - d * E, p = e * DP + d;
   if (NC * T1 == NT || tid < NC * T1) {
     const int team = tid / T1, t = tid - team * T1, c = c0 + team;
     const float2* Ic = I + ((size_t)(b0 + e) * HS + c) * L + t;
@@ -98,6 +100,7 @@ __global__ void __launch_bounds__(col_threads<L, NC>(), MINB)
   __syncthreads();
   if (chained) griddep_wait();  // Q is still being read by the previous row pass
   const int col = tid % NC, j0 = tid / NC;
+  const unsigned long long keep = l2_keep_policy();
   const unsigned flip = c0 + col ? 0x80000000u : 0u;  // column -kx: the conjugate
   float4* Qp = Q + (size_t)p * NZ * L + c0 + col;
 #pragma unroll
@@ -116,9 +119,11 @@ __global__ void __launch_bounds__(col_threads<L, NC>(), MINB)
     for (int r = 0; r < R2 / 2; ++r) {
       const Cx2 u = x[r], w = x[r + R2 / 2];
       float4* o = Qp + (size_t)(j + r * R1) * L;
-      o[0] = make_float4(u.re.x, u.im.x, w.re.x, w.im.x);
-      o[NZ] = make_float4(u.re.y, __uint_as_float(__float_as_uint(u.im.y) ^ flip), w.re.y,
-                          __uint_as_float(__float_as_uint(w.im.y) ^ flip));
+      store_hint(o, make_float4(u.re.x, u.im.x, w.re.x, w.im.x), keep);
+      store_hint(o + NZ,
+                 make_float4(u.re.y, __uint_as_float(__float_as_uint(u.im.y) ^ flip), w.re.y,
+                             __uint_as_float(__float_as_uint(w.im.y) ^ flip)),
+                 keep);
     }
   }
 }
@@ -130,9 +135,11 @@ __global__ void __launch_bounds__(col_threads<L, NC>(), MINB)
 // double-buffered stream of bulk copies (a row pair of Q is one contiguous block) on its own
 // mbarriers, with no barrier of the CTA between pairs.  Every wait is bounded: on timeout the
 // team raises *a.err and fetches no further rows.
-// Q is dead once it has been read: each row pair's lines are discarded from L2, from where the next
-// column pass would otherwise write them back to DRAM (a 4096^2 search at window 512: 321 -> 311 ms;
-// at window 320 no difference).
+// Q, 160 MB per launch, passes through an L2 that keeps about 35 MB of it.  The pairs are taken in
+// descending order, the last written (whose stores ask to be kept) first; and each row pair's lines,
+// dead once read, are discarded from L2, from where the next column pass would otherwise write them
+// back to DRAM.  A 4096^2 search at window 512: 321 -> 311 ms by the discarding, -> 304 ms by the
+// order and the stores' hint (the order alone: half of that).
 template <int L, int RB, int DS, int EPI, int MINB>
 __global__ void __launch_bounds__(2 * RowPlan2<L>::T* RB* DS, MINB)
     pair_rows_kernel(CorrArgs a, const float2* __restrict__ twL) {
@@ -150,7 +157,7 @@ __global__ void __launch_bounds__(2 * RowPlan2<L>::T* RB* DS, MINB)
   const int row = team % RB, s = team / RB;
   const int e = blockIdx.y, y = blockIdx.x * RB + row, win = a.b0 + e;
   const int angle = a.angle_state ? a.angle_state->index : a.angle;
-  const int DP = (a.D + 1) / 2, np = (DP - s + DS - 1) / DS;  // this team's pairs s, s + DS, ...
+  const int DP = (a.D + 1) / 2, np = (DP - s + DS - 1) / DS;  // this team's pairs s, s + DS, ..., from the last
   float2* buf = stage + (size_t)team * 2 * PAIR;
   if (u == 0) {
     mbar_init(&bars[team][0], 1);
@@ -168,7 +175,7 @@ __global__ void __launch_bounds__(2 * RowPlan2<L>::T* RB* DS, MINB)
 #pragma unroll
   for (int i = 0; i < E; ++i) {
     s2[i] = 0.f;
-    if constexpr (BEST) best[i] = -INFINITY;
+    if constexpr (BEST) best[i] = TOPK ? -FLT_MAX : -INFINITY;
     if constexpr (TOPK) barg[i / 2] = 0u;
   }
   const float inv = 1.0f / (float)(L * L);
@@ -178,7 +185,7 @@ __global__ void __launch_bounds__(2 * RowPlan2<L>::T* RB* DS, MINB)
   constexpr unsigned kBytes = L * (unsigned)sizeof(float4);
   static_assert(kBytes % 128 == 0, "whole lines");
   auto row_pair = [&](int k) {
-    return reinterpret_cast<const float4*>(a.Q) + ((size_t)(e * DP + s + DS * k) * (L / 2) + y) * L;
+    return reinterpret_cast<const float4*>(a.Q) + ((size_t)(e * DP + s + DS * (np - 1 - k)) * (L / 2) + y) * L;
   };
   auto issue = [&](int k) {
     fence_proxy_async_smem();
@@ -198,7 +205,7 @@ __global__ void __launch_bounds__(2 * RowPlan2<L>::T* RB* DS, MINB)
       ok = mbar_wait(&bars[team][k & 1], (k >> 1) & 1, 4000000000LL);
       failed = k;
     }
-    const int d = 2 * (s + DS * k);
+    const int d = 2 * (s + DS * (np - 1 - k));
     const bool two = d + 1 < a.D;  // an odd template count leaves the last pair half empty
     float m1 = -INFINITY, m2 = -INFINITY;
     float2* in = buf + (k & 1) * PAIR + h;  // element i of this thread's row at 2 i
@@ -206,11 +213,7 @@ __global__ void __launch_bounds__(2 * RowPlan2<L>::T* RB* DS, MINB)
     float2 v[E];
 #pragma unroll
     for (int m = 0; m < E; ++m) v[m] = in[2 * (m < E / 2 ? t + T * m : m == E / 2 ? mid : up - T * m)];
-    if (ok) {  // the row pair has been copied: what of it is still in L2 need not be written back
-      const char* src = reinterpret_cast<const char*>(row_pair(k));
-      for (int i = u; i < (int)kBytes / 128; i += TT)
-        asm volatile("discard.global.L2 [%0], 128;" ::"l"(src + 128 * i) : "memory");
-    }
+    if (ok) discard_lines(row_pair(k), kBytes, u, TT);  // (the row pair has been copied)
     team_sync<TT>(team);
     RegDft<float2, R1, +1>::run(v);
 #pragma unroll
@@ -257,14 +260,14 @@ __global__ void __launch_bounds__(2 * RowPlan2<L>::T* RB* DS, MINB)
           m1 = fmaxf(m1, c1);
           m2 = fmaxf(m2, cm);
         }
-        if constexpr (TOPK) {
-          if (c1 > best[i]) {
-            best[i] = c1;
-            put_half(barg[i / 2], i & 1, d + 1);
-          }
-          if (two && c2 > best[i]) {
+        if constexpr (TOPK) {  // (templates in descending order: equal values keep the lowest)
+          if (two && c2 >= best[i]) {
             best[i] = c2;
             put_half(barg[i / 2], i & 1, d + 2);
+          }
+          if (c1 >= best[i]) {
+            best[i] = c1;
+            put_half(barg[i / 2], i & 1, d + 1);
           }
         }
       }
@@ -312,7 +315,7 @@ __global__ void __launch_bounds__(2 * RowPlan2<L>::T* RB* DS, MINB)
           const float b = o[(E + i) * TT];
           const unsigned g2 = __float_as_uint(o[(2 * E + i / 2) * TT]);
           const unsigned g = i & 1 ? g2 >> 16 : g2 & 0xFFFFu, own = i & 1 ? barg[i / 2] >> 16 : barg[i / 2] & 0xFFFFu;
-          if (g && (b > best[i] || (b == best[i] && g < own))) {
+          if (g && (b > best[i] || (b == best[i] && (g < own || !own)))) {
             best[i] = b;
             put_half(barg[i / 2], i & 1, (int)g);
           }
