@@ -142,7 +142,8 @@ typedef struct gisspa_stats {
   double templates_per_launch; /* mean template batch depth D per launch of the search */
   int pass_samples;
   int window_size;
-  int pass_b_variant;          /* pass B shape picked by the autotuner (last sweep); at window 512
+  int pass_b_variant;          /* pass B shape picked by the autotuner (last sweep that it tuned:
+                                  a first sweep with two templates per transform is not); at window 512
                                   shape 4 is the pair engine (both passes in one launch) */
   double tuned_us_per_pair;    /* autotuner's measured time per pair of that shape */
   long long graph_replays;     /* angles run as replays of a captured CUDA graph */
