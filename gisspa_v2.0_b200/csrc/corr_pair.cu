@@ -14,7 +14,8 @@
 // Measured on B200 (window 512, FP32, 24 templates x 6 windows per launch, 1.9 GHz): 0.60 us per
 // (window, template) correlation, column pass 0.34, row pass 0.26, against 0.83 for the
 // one-template passes (correlate.cu); a 4096^2 search with 40 templates 393 instead of 518 ms,
-// 1855 x 1919 at window 320 37 instead of 54 ms.  The column pass is bound by L2 traffic (1.5 MB
+// 1855 x 1919 at window 320 37 instead of 54 ms (0.58 us with the order in which Q is read, see the
+// row pass; 1.7 us at window 1024 instead of 2.5).  The column pass is bound by L2 traffic (1.5 MB
 // of spectra read and 1 MB of Q written per correlation; without its stores it takes 0.20, with
 // a Q of 32 MB that stays in L2 0.26), the row pass by latency at 12 warps per SM (61 % of
 // issue slots; 552 instructions per row and template pair against 1090).
@@ -439,6 +440,7 @@ template <int L>
 struct PairShape;
 template <> struct PairShape<256> { static constexpr int NC = 8, MA = 4, RB = 2, WARPS = 16; };
 template <> struct PairShape<320> { static constexpr int NC = 8, MA = 3, RB = 2, WARPS = 16; };
+template <> struct PairShape<1024> { static constexpr int NC = 4, MA = 3, RB = 1, WARPS = 12; };
 template <> struct PairShape<512> { static constexpr int NC = 8, MA = 3, RB = 1, WARPS = 12; };
 
 template <int L, typename SPEC>
@@ -466,12 +468,12 @@ void rows_ds(const CorrLaunch& cl, const CorrArgs& a, const float2* twL, cudaStr
   launch_pdl(kernel, dim3(L / 2 / S::RB, cl.E), dim3(threads), smem, s, a, twL);
 }
 
-// Shares per row pair: a launch has L / 2 x E row pairs, each a warp's serial chain over the
+// Shares per row pair: a launch has L / 2 x E row pairs, each a team's serial chain over the
 // template pairs; where that leaves half or more of the chip's warp slots empty the chains are
 // cut in two or three.
 template <int L, int EPI>
 void rows(const CorrLaunch& cl, const CorrArgs& a, const float2* twL, cudaStream_t s) {
-  const int slots = 148 * PairShape<L>::WARPS, chains = L / 2 * cl.E, pairs = (cl.D + 1) / 2;
+  const int slots = 148 * PairShape<L>::WARPS / (RowPlan2<L>::T / 16), chains = L / 2 * cl.E, pairs = (cl.D + 1) / 2;
   const int ds = std::min(slots / chains, pairs);
   if (ds >= 3 && PairShape<L>::RB == 1)
     rows_ds<L, EPI, PairShape<L>::RB == 1 ? 3 : 2>(cl, a, twL, s);
@@ -502,16 +504,21 @@ void launch(const CorrLaunch& cl, const float2* I, const void* T, float2* Q, con
 }  // namespace
 
 bool pair_supported(int L, int epi) {
-  return (L == 256 || L == 320 || L == 512) && (epi == EPI_SUM || epi == EPI_SUMMAX || epi == EPI_TOPK);
+  return (L == 256 || L == 320 || L == 512 || L == 1024) && (epi == EPI_SUM || epi == EPI_SUMMAX || epi == EPI_TOPK);
 }
 
-// Windows and templates per launch.  E fills the row pass's warp slots with one chain per row
+// Windows and templates per launch.  E fills the row pass's team slots with one chain per row
 // pair; D then makes the state's reductions (12 bytes per pixel and launch) small beside the D/2
-// row pairs of Q they stand for, with at most 160 MB of Q.
+// row pairs of Q they stand for, with at most 160 MB of Q.  At window 1024 one window's chains fill
+// 0.58 of the slots and three's 1.73 (two rounds, 0.86): three windows and 240 MB of Q, evened out
+// over the windows (a 3838 x 3710 search: 85.8 ms; 1 window x 20 templates 105, 3 x 10 88.9, 5 x 16
+// 91.7; one-template passes 116).
 void pair_batch(int L, int W, int nt, int& D, int& E) {
-  const int slots = 148 * (L == 512 ? 12 : 16);
-  E = std::max(1, std::min(W, slots / (L / 2)));
-  const long long cap = (160LL << 20) / ((long long)L * L * 4) / E;
+  if (L == 1024)
+    E = ceil_div(W, ceil_div(W, 3));
+  else
+    E = std::max(1, std::min(W, 148 * (L == 512 ? 12 : 16) / (L / 2)));
+  const long long cap = ((L == 1024 ? 240LL : 160LL) << 20) / ((long long)L * L * 4) / E;
   D = (int)std::min<long long>(std::max<long long>(cap, 2), kMaxListedTemplates) & ~1;
   const int n = (nt + D - 1) / D;  // launches per window batch, evened out
   D = ((nt + n - 1) / n + 1) & ~1;
@@ -569,6 +576,7 @@ void pair_launch(const CorrLaunch& cl, const float2* I, const void* T, float2* Q
     case 256: launch<256>(cl, I, T, Q, args, twL, s, ev); break;
     case 320: launch<320>(cl, I, T, Q, args, twL, s, ev); break;
     case 512: launch<512>(cl, I, T, Q, args, twL, s, ev); break;
+    case 1024: launch<1024>(cl, I, T, Q, args, twL, s, ev); break;
     default: throw CudaError{cudaErrorInvalidValue, "window size without paired correlation kernels"};
   }
 }

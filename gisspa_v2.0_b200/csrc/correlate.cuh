@@ -147,7 +147,7 @@ void engine_launch(int spec, int epi, const float2* I, const void* T, const Engi
                    cudaStream_t s);
 
 // ---- sweep 1 with two templates per transform (corr_pair.cu): EPI_SUM, EPI_SUMMAX and EPI_TOPK
-// at window sizes 256, 320 and 512.  Adds the sums of squares and the maxima to the state; the
+// at window sizes 256, 320, 512 and 1024.  Adds the sums of squares and the maxima to the state; the
 // plain sums come from pair_sum_finish.  Several angles can go through one launch: "template"
 // v = a nt + t is template t at the a-th of them (args.angle or angle_state: the first).
 bool pair_supported(int L, int epi);

@@ -637,12 +637,13 @@ bool sweep_paired(const gisspa_config& cfg, int l, int epi) {
          !(cfg.tensor_cores && cfg.spectrum_precision == GISSPA_SPEC_FP16 && l == 512);
 }
 
-// Angles per step of a paired sweep over n angles: up to 256 rotated templates together, so that a
-// few templates or windows still fill the GPU and a launch's fixed costs (each of the step's kernels
-// takes 4 to 15 us however small) are shared; at least three steps, the last ones replays of a graph.
+// Angles per step of a paired sweep over n angles: up to 256 rotated templates (64 of window 1024)
+// together, so that a few templates or windows still fill the GPU and a launch's fixed costs (each
+// of the step's kernels takes 4 to 15 us however small) are shared; at least three steps, the last
+// ones replays of a graph.
 // A divisor of n where one is near.
-int angles_per_step(int nt, int n) {
-  const int most = std::max(1, std::min(kMaxListedTemplates / nt, n / 3));
+int angles_per_step(int l, int nt, int n) {
+  const int most = std::max(1, std::min((l == 1024 ? 64 : kMaxListedTemplates) / nt, n / 3));
   for (int na = most; 2 * na > most; --na)
     if (n % na == 0) return na;
   return most;
@@ -1009,7 +1010,7 @@ void run_angles(Ctx& c, NormRun& r, int epi, int a0, int a1) {
   gisspa_handle* h = c.h;
   if (a1 <= a0) return;
   const bool paired = sweep_paired(h->cfg, c.l, epi);
-  const int na = paired ? angles_per_step(h->nt, a1 - a0) : 1, steps = (a1 - a0) / na;
+  const int na = paired ? angles_per_step(c.l, h->nt, a1 - a0) : 1, steps = (a1 - a0) / na;
   const bool graphs = h->cfg.cuda_graphs != 0 && steps >= 3;
   AngleState* table = buf<AngleState>(h->angle_table, r.angles.size());
   if ((graphs || paired) && !r.angle_table_ready) {

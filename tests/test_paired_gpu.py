@@ -1,4 +1,4 @@
-"""Sweep 1 with two templates per transform (window sizes 256, 320, 512) against the one-template
+"""Sweep 1 with two templates per transform (window sizes 256, 320, 512, 1024) against the one-template
 kernels that a fixed launch shape selects: per-pixel sums, sums of squares and best correlations
 of one rank's sweep.  Template counts that leave the last pair half empty or a launch with fewer
 pairs than shares per row, one window and several, every spectrum precision."""
@@ -11,7 +11,7 @@ import synth
 pytestmark = pytest.mark.gpu
 
 # Both paths hold the same stored spectra and FP32 transforms of 2 L^2 points: either's rounding is
-# at most about log2(L^2) * 2^-24 = 1.1e-6 of the map's rms (L = 512); ten times that bounds the
+# at most about log2(L^2) * 2^-24 = 1.2e-6 of the map's rms (L = 1024); ten times that bounds the
 # difference of sums over a few dozen of them.
 RTOL = 1e-5
 
@@ -37,7 +37,8 @@ def _state(cfg, tmpl, img, ctf):
 @pytest.mark.parametrize("spec", [gisspa.SPEC_FP32, gisspa.SPEC_FP16, gisspa.SPEC_BF16])
 @pytest.mark.parametrize("L,shape,nt", [(256, (256, 256), 1), (256, (500, 700), 7), (320, (320, 320), 2),
                                         (320, (500, 660), 5), (512, (512, 512), 9), (512, (512, 512), 3),
-                                        (512, (900, 1300), 4)])
+                                        (512, (900, 1300), 4), (1024, (1024, 1024), 3),
+                                        (1024, (1900, 2700), 4)])
 def test_paired_sweep_equals_the_one_template_sweep(L, shape, nt, spec):
     c = synth.make_case(shape=shape, n_particles=3, snr=0.5, n_templates=nt, tsize=L // 4, seed=L + nt, margin=L // 5)
     cfg = gisspa.Config.default(angpix=1.0, phistep=60.0, kk=3.0, energy=300.0, cs=2.7, highres=8.0, lowres=200.0,
