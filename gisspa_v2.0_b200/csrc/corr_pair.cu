@@ -136,8 +136,8 @@ __global__ void __launch_bounds__(col_threads<L, NC>(), MINB)
 // double-buffered stream of bulk copies (a row pair of Q is one contiguous block) on its own
 // mbarriers, with no barrier of the CTA between pairs.  Every wait is bounded: on timeout the
 // team raises *a.err and fetches no further rows.
-// Q, 160 MB per launch, passes through an L2 that keeps about 35 MB of it.  The pairs are taken in
-// descending order, the last written (whose stores ask to be kept) first; and each row pair's lines,
+// Q, 160 MB per launch, passes through an L2 that kept 33 MB of it.  The pairs are taken in descending
+// order, the last written (whose stores ask to be kept) first: 57 MB; and each row pair's lines,
 // dead once read, are discarded from L2, from where the next column pass would otherwise write them
 // back to DRAM.  A 4096^2 search at window 512: 321 -> 311 ms by the discarding, -> 304 ms by the
 // order and the stores' hint (the order alone: half of that).
